@@ -119,6 +119,68 @@ __device__ __forceinline__ void sincos_half64(double x, double *s, double *c) {
     sincos_poly64(x, ps, pc, s, c);
 }
 
+// Offsets from a reduced phase or amplitude, with a bound on |x| known to the caller as an offset class:
+// 1: |x| <= 3/4, 2: |x| <= 3/8, 0: none.  Chebyshev coefficients (fit_sincos.py, highest degree first);
+// maximum absolute errors of sin / cos: class 1 5.3e-18 / 5.2e-19, class 2 1.3e-18 / 3.2e-17; of exp, as
+// e^x = 1 + x E(x), relative: 3.2e-18 and 2.6e-17.  FP64 operations: 15 and 12 for the pair (sincos_cw64
+// takes 20 and two selections), 14 and 11 for exp.
+#define BC_SIN_OFF1 {1.5930497086426094e-10, -2.5051295945987136e-08, 2.7557316855764324e-06, \
+                     -0.00019841269838148635, 0.00833333333333183, -0.16666666666666666}
+#define BC_COS_OFF1 {-1.1377016289560215e-11, 2.087603297418857e-09, -2.755731644892395e-07, \
+                     2.480158729612574e-05, -0.001388888888888377, 0.04166666666666665, -0.5}
+#define BC_SIN_OFF2 {-2.499571220213754e-08, 2.7557249854310547e-06, -0.00019841269806435577, \
+                     0.008333333333327211, -0.16666666666666666}
+#define BC_COS_OFF2 {-2.7484016455684523e-07, 2.480149714091543e-05, -0.0013888888843615426, \
+                     0.04166666666658709, -0.4999999999999998}
+#define BC_EXP_OFF1 {1.156521003382576e-11, 1.6210260812877196e-10, 2.0876025433715686e-09, 2.505093714055246e-08, \
+                     2.75573220313723e-07, 2.7557323719055684e-06, 2.48015872960584e-05, 0.0001984126983241682, \
+                     0.0013888888888894074, 0.008333333333341636, 0.04166666666666665, 0.16666666666666638, 0.5, 1.0}
+#define BC_EXP_OFF2 {2.5114284550153316e-08, 2.7638162815097353e-07, 2.7557231755822327e-06, 2.4801473565882206e-05, \
+                     0.00019841269895092592, 0.0013888888958877, 0.008333333333319816, 0.041666666666490895, \
+                     0.16666666666666677, 0.5000000000000012, 1.0}
+
+template <int CLS>
+__device__ __forceinline__ void sincos_off64(double x, double *s, double *c) {
+    if constexpr (CLS == 1) {
+        constexpr double ps[] = BC_SIN_OFF1;
+        constexpr double pc[] = BC_COS_OFF1;
+        sincos_poly64(x, ps, pc, s, c);
+    } else if constexpr (CLS == 2) {
+        constexpr double ps[] = BC_SIN_OFF2;
+        constexpr double pc[] = BC_COS_OFF2;
+        sincos_poly64(x, ps, pc, s, c);
+    } else {
+        sincos_cw64(x, s, c);
+    }
+}
+
+// Horner evaluation of e^x = 1 + x E(x).
+template <int N>
+__device__ __forceinline__ double exp_poly64(double x, const double (&pe)[N]) {
+    double p = pe[0];
+#pragma unroll
+    for (int i = 1; i < N; ++i) p = fma(p, x, pe[i]);
+    return fma(p, x, 1.0);
+}
+
+template <int CLS>
+__device__ __forceinline__ double exp_off64(double x) {
+    if constexpr (CLS == 1) {
+        constexpr double pe[] = BC_EXP_OFF1;
+        return exp_poly64(x, pe);
+    } else if constexpr (CLS == 2) {
+        constexpr double pe[] = BC_EXP_OFF2;
+        return exp_poly64(x, pe);
+    } else {
+        return exp(x);
+    }
+}
+
+// The offset class of a bound on |x| (0: unknown or large).
+inline int offset_class64(double bound) {
+    return !(bound > 0.0) ? 0 : bound <= 0.375 ? 2 : bound <= 0.75 ? 1 : 0;
+}
+
 // |x| <= 1/2 in FP32: degree 5 (sin) and 6 (cos), BC_*_HALF32.
 __device__ __forceinline__ void sincos_half32(float x, float *s, float *c) {
     constexpr float ps[] = BC_SIN_HALF32;

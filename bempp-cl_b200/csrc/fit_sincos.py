@@ -3,10 +3,11 @@
 Method: Chebyshev approximation (mpmath.chebyfit, 50 significant digits) of
     g(t) = (sin(sqrt t) - sqrt t) / t^(3/2)   so that sin x = x + x^3 P(x^2),
     h(t) = (cos(sqrt t) - 1) / t              so that cos x = 1 + x^2 Q(x^2),
-on t in [0, a^2] for the three argument ranges used by the kernels:
+on t in [0, a^2] for the argument ranges used by the kernels:
     a = 1/2   (sincos_half64: phase offsets |k| (R_i + R_j) <= 1/2)
     a = 1     (sincos_small64: offsets <= 1)
-    a = pi/4  (sincos_cw64: after Cody-Waite reduction).
+    a = pi/4  (sincos_cw64: after Cody-Waite reduction)
+    a = 3/4, 3/8  (sincos_off64: phase offsets by class; exp_off64 for amplitudes).
 The coefficients are rounded to double; the script prints them (highest degree
 first, as the Horner loops consume them) with the maximum absolute error of the
 rounded polynomial against the 50-digit function over 4001 points of [0, a].
@@ -33,7 +34,11 @@ import numpy as np
 mp.mp.dps = 50
 
 # (name, a, number of sine coefficients, number of cosine coefficients)
-CLASSES = (("half64", mp.mpf(1) / 2, 5, 6), ("small64", mp.mpf(1), 7, 7), ("cw64", mp.pi / 4, 6, 7))
+CLASSES = (("half64", mp.mpf(1) / 2, 5, 6), ("small64", mp.mpf(1), 7, 7), ("cw64", mp.pi / 4, 6, 7),
+           ("off1", mp.mpf(3) / 4, 6, 7), ("off2", mp.mpf(3) / 8, 5, 5))
+
+# (name, a, number of coefficients) of e^x = 1 + x E(x) on |x| <= a, E by Chebyshev approximation
+EXP_CLASSES = (("off1", mp.mpf(3) / 4, 14), ("off2", mp.mpf(3) / 8, 11))
 
 
 def _g(t):
@@ -61,6 +66,20 @@ def fit(kind, a, ncoeff):
             p = p * t + mp.mpf(c)
         v, ref = (x + x**3 * p, mp.sin(x)) if kind == "sin" else (1 + t * p, mp.cos(x))
         worst = max(worst, abs(v - ref))
+    return coeffs, float(worst)
+
+
+def fit_exp(a, ncoeff):
+    """Coefficients of E and the maximum relative error of 1 + x E(x) on [-a, a]."""
+    poly = mp.chebyfit(lambda t: mp.expm1(t) / t if t != 0 else mp.mpf(1), [-a, a], ncoeff)
+    coeffs = [float(c) for c in poly]
+    worst = mp.mpf(0)
+    for i in range(4001):
+        x = -a + 2 * a * i / 4000
+        p = mp.mpf(0)
+        for c in coeffs:
+            p = p * x + mp.mpf(c)
+        worst = max(worst, abs((1 + x * p) / mp.exp(x) - 1))
     return coeffs, float(worst)
 
 
@@ -114,6 +133,9 @@ if __name__ == "__main__":
         for kind, n in (("sin", ns), ("cos", nc)):
             coeffs, err = fit(kind, a, n)
             print("%s %s (max abs error %.2e): {%s}" % (name, kind, err, ", ".join(repr(c) for c in coeffs)))
+    for name, a, n in EXP_CLASSES:
+        coeffs, err = fit_exp(a, n)
+        print("%s exp (max relative error %.2e): {%s}" % (name, err, ", ".join(repr(c) for c in coeffs)))
     for name, a, ns, nc in CLASSES32:
         for kind, n in (("sin", ns), ("cos", nc)):
             coeffs = fit32(kind, a, n)

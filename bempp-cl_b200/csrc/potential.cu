@@ -10,15 +10,19 @@
 //  1. potential_sources: one thread per (element, quadrature point) writes the
 //     source point, normal and weighted coefficient(s) field-major into the
 //     caller's workspace (the reference's `tmp` arrays).
-//  2. potential_scalar (Laplace, Helmholtz and modified Helmholtz single /
+//  2. the mixed-precision kernels, or for FP64 with a rule that is not made of
+//     two orbits (any order but 4):
+//     potential_scalar (Laplace, Helmholtz and modified Helmholtz single /
 //     double layer): a thread per evaluation point walks the sources staged
 //     in shared memory; see the comment above the kernel.
 //     potential_eval (far fields, Maxwell): one warp owns PPW evaluation points;
 //     its lanes stride over the sources with coalesced loads, accumulate per
 //     point in FP64 and combine with xor-shuffle reductions; lane 0 writes.
+// FP64 with the order-4 rule takes potential_orbit.cuh instead of both.
 #include <algorithm>
 
 #include "dp0.cuh"  // common.cuh, and the packed FP32 helpers of the mixed kernels
+#include "potential.cuh"
 
 namespace bc {
 
@@ -28,23 +32,6 @@ namespace bc {
 constexpr int SRC_FIELDS = 14;
 constexpr int POT_PPW = 4;
 constexpr int POT_WARPS = 4;
-
-struct PotParams {
-    const double *g;
-    int64_t ne;
-    const uint32_t *support;
-    int64_t nsupport;
-    const int32_t *nm;
-    int nshape;
-    int nq;
-    const double *coeff;  // complex (ne * nshape)
-    double *src;          // workspace SRC_FIELDS * nsrc
-    int64_t nsrc;
-    const double *points;  // (npoints, 3)
-    int64_t npoints;
-    double *result;  // complex (kdim, npoints)
-    double p[4];
-};
 
 template <bool MAXWELL>
 __global__ void potential_sources(PotParams prm, QuadRule rule) {
@@ -279,7 +266,7 @@ __device__ __forceinline__ void phase_small(double t, double *s, double *c) {
 // PHC 0-2: real wavenumber (1, 2: factored about the element centroid); PHC 3: complex wavenumber
 // k = kr + i ki, exp(i kr r) exp(-ki r) per point-source pair and (ikr - 1) = -(1 + ki r) + i kr r.
 // Modified Helmholtz (real kernel, w = p[0]): the Laplace kernels times exp(-w r) or exp(-w r) (1 + w r).
-template <int K, int PHC, int NQ>
+template <int K, int PHC>
 __global__ void __launch_bounds__(PS_THREADS) potential_scalar(PotParams prm, int64_t chunk_elems) {
     constexpr bool HELM = (K == BEMPPCUDA_HELMHOLTZ_SLP || K == BEMPPCUDA_HELMHOLTZ_DLP);
     constexpr bool MH = (K == BEMPPCUDA_MODHELM_SLP || K == BEMPPCUDA_MODHELM_DLP);
@@ -288,7 +275,7 @@ __global__ void __launch_bounds__(PS_THREADS) potential_scalar(PotParams prm, in
     constexpr bool CK = HELM && PHC == 3;
     __shared__ double2 ssrc[PS_SOURCES * 4];        // {y0 y1} {y2 cre} {cim n0} {n1 n2}
     __shared__ double2 scen[FACTOR ? PS_SOURCES * 2 : 2];  // {c0 c1} {c2 -} per element
-    const int nq = NQ ? NQ : prm.nq;
+    const int nq = prm.nq;
     const int tile_elems = PS_SOURCES / nq;
     const int64_t ebeg = (int64_t)blockIdx.y * chunk_elems;
     const int64_t eend = min(ebeg + chunk_elems, prm.nsupport);
@@ -1188,7 +1175,7 @@ static cudaError_t scalar_grid(const PotParams &prm, const void *fn, dim3 *grid,
 
 template <int K, int PHC>
 static cudaError_t launch_scalar_nq(const PotParams &prm, cudaStream_t st) {
-    auto fn = prm.nq == 6 ? potential_scalar<K, PHC, 6> : potential_scalar<K, PHC, 0>;
+    auto fn = potential_scalar<K, PHC>;
     dim3 grid;
     int64_t chunk_elems = 0;
     const cudaError_t err = scalar_grid(prm, (const void *)fn, &grid, &chunk_elems, st);
@@ -1389,7 +1376,11 @@ int bc_potential_launch(const bemppcuda_potential_args *a, double *workspace, cu
         return BEMPPCUDA_ERR_INVALID;
     }
     if (prm.npoints == 0) return BEMPPCUDA_OK;
-    if (prm.nsrc > 0) {
+    // FP64 with the two-orbit six-point rule (the order-4 rule): potential_orbit.cuh
+    OrbitRule orbit;
+    const bool orbits = !mixed && prm.nsupport > 0 && orbit_rule(rule, orbit) &&
+                        potential_orbit_has(a->assembly, a->kernel);
+    if (prm.nsrc > 0 && !orbits) {
         const unsigned blocks = (unsigned)((prm.nsrc + 255) / 256);
         if (maxwell)
             potential_sources<true><<<blocks, 256, 0, st>>>(prm, rule);
@@ -1397,7 +1388,9 @@ int bc_potential_launch(const bemppcuda_potential_args *a, double *workspace, cu
             potential_sources<false><<<blocks, 256, 0, st>>>(prm, rule);
     }
     cudaError_t err = cudaGetLastError();
-    if (err == cudaSuccess) {
+    if (err == cudaSuccess && orbits) {
+        err = launch_potential_orbit(prm, orbit, a->assembly, a->kernel, a->phase_radius, st);
+    } else if (err == cudaSuccess) {
         const bool per_point = a->kernel == BEMPPCUDA_LAPLACE_SLP || a->kernel == BEMPPCUDA_LAPLACE_DLP ||
                                a->kernel == BEMPPCUDA_HELMHOLTZ_SLP || a->kernel == BEMPPCUDA_HELMHOLTZ_DLP ||
                                a->kernel == BEMPPCUDA_MODHELM_SLP || a->kernel == BEMPPCUDA_MODHELM_DLP;
