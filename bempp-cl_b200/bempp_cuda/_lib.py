@@ -309,6 +309,7 @@ SIGNATURES = {
                                                 _vp]),
     "bemppcuda_project": (_ct.c_int, [_ct.POINTER(GridRec), _ct.POINTER(Space), _i32, _vp, _vp, _vp, _vp, _vp]),
     "bemppcuda_assemble_singular": (_ct.c_int, [_ct.POINTER(SingularArgs), _vp]),
+    "bemppcuda_assemble_singular_duffy": (_ct.c_int, [_ct.POINTER(SingularArgs), _ct.c_int32, _vp]),
     "bemppcuda_potential_workspace_bytes": (_i64, [_ct.POINTER(PotentialArgs)]),
     "bemppcuda_evaluate_potential": (_ct.c_int, [_ct.POINTER(PotentialArgs), _vp]),
     "bemppcuda_fma_probe": (_ct.c_int, [_i32, _i64, _i64, _vp, _ct.POINTER(_ct.c_double), _vp]),
@@ -316,6 +317,7 @@ SIGNATURES = {
     "bemppcuda_batch_workspace_bytes": (_i64, [_i32]),
     "bemppcuda_batch_prepare": (_ct.c_int, [_ct.POINTER(BatchArgs), _vp]),
     "bemppcuda_batch_launch": (_ct.c_int, [_ct.POINTER(BatchArgs), _vp]),
+    "bemppcuda_batch_launch_duffy": (_ct.c_int, [_ct.POINTER(BatchArgs), _ct.c_int32, _vp]),
     "bemppcuda_assemble_identity": (_ct.c_int, [_ct.POINTER(IdentityArgs), _vp]),
     "bemppcuda_matmat_workspace_bytes": (_i64, [_i32]),
     "bemppcuda_matmat_prepare": (_ct.c_int, [_ct.POINTER(MatmatArgs), _vp]),

@@ -268,6 +268,15 @@ def dp0_fast_path(descriptor, domain, dual_to_range, parameters):
     return bool(device_space(domain).dof_is_position and device_space(dual_to_range).dof_is_position)
 
 
+def _same_maps(domain, dual_to_range, assembly):
+    """True for the Maxwell fields on spaces with equal supports and dof maps (RWG and SNC of one grid): the device
+    copies are then shared, and the operators are symmetric under exchanging a pair's elements."""
+    if assembly not in (_lib.ASM_EFIE, _lib.ASM_MFIE):
+        return False
+    a, b = device_space(domain), device_space(dual_to_range)
+    return a.support is b.support and a.l2g is b.l2g and a.mult is b.mult
+
+
 def singular_into_dense(result, descriptor, domain, dual_to_range, parameters, diag_shift=0.0, stream=None,
                         geometry=None, rows=None, mirror=True):
     """Scatter the Sauter-Schwab pairs into the dense device tensor ``result`` (``geometry`` as in regular_into).
@@ -301,14 +310,14 @@ def singular_into_dense(result, descriptor, domain, dual_to_range, parameters, d
     args.ld = result.stride(0)
     args.diag_shift = float(diag_shift)
     args.phase_radius = 1.0001 * 2.0 * (geometry or device_grid(grid)).radius
-    if mirror and same_space(domain, dual_to_range):
+    order = int(parameters.quadrature.singular)
+    if mirror and (same_space(domain, dual_to_range) or _same_maps(domain, dual_to_range, assembly)):
         # every pair is listed in both orders and the vertex-adjacent rule (its weights follow the
-        # coincident and edge-adjacent ones) is symmetric in test and trial points: the DP0 kernel
-        # evaluates each such pair once for both entries
-        order = parameters.quadrature.singular
+        # coincident and edge-adjacent ones) is symmetric in test and trial points: each such pair is
+        # evaluated once for both entries
         args.mirror_weights_offset = (number_of_duffy_points(order, "coincident")
                                       + number_of_duffy_points(order, "edge_adjacent"))
-    _lib.check(_lib.load().bemppcuda_assemble_singular(args, stream or current_stream()))
+    _lib.check(_lib.load().bemppcuda_assemble_singular_duffy(args, order, stream or current_stream()))
     return result
 
 

@@ -66,6 +66,7 @@ class BatchAssembler(object):
         if int(order_reg) != 4:
             raise ValueError("the batched kernel uses the 6-point rule (regular order 4)")
         self.kernel = kernel
+        self._order = int(order_sing)
         self.grids = list(grids)
         self.wavenumbers = [complex(k) for k in wavenumbers]
         self.precisions = precisions
@@ -144,7 +145,7 @@ class BatchAssembler(object):
         _lib.check(_lib.load().bemppcuda_batch_prepare(_ct.byref(self.args), current_stream()))
 
     def launch(self):
-        _lib.check(_lib.load().bemppcuda_batch_launch(_ct.byref(self.args), current_stream()))
+        _lib.check(_lib.load().bemppcuda_batch_launch_duffy(_ct.byref(self.args), self._order, current_stream()))
 
     def set_shape(self, rows_per_item, blocks_per_sm):
         self.args.rows_per_item = int(rows_per_item)

@@ -9,8 +9,12 @@
 // launch over the concatenated pair list (FP64).
 #include <cstring>
 
+#include <algorithm>
+#include <type_traits>
+
 #include "dp0_sym.cuh"
 #include "singular_dp0.cuh"
+#include "singular_duffy.cuh"
 
 namespace bc {
 
@@ -24,7 +28,7 @@ struct BatchDev {
     int32_t precision;
     int32_t phase_class;
     int32_t ck;
-    int32_t pad;
+    int32_t sing_class;  // offset class of the touching pairs
     double diag_shift;
 };
 
@@ -214,6 +218,73 @@ static int64_t tiles_of(int64_t n, int rows, bool sym) {
     return sym_tiles_before(tx - 1, g) + (ty < g * tx ? ty : g * tx);
 }
 
+// The touching pairs of all problems on the order-4 rules (singular_duffy.cuh), 8 lanes per pair; a warp's four
+// pairs, which mostly belong to one problem, share the least of their offset classes (CK: some problem has a complex
+// wavenumber; a real one is then complex with Im k = 0).  Each pair is listed in both orders, so the
+// vertex-adjacent pair t < s adds both entries.
+template <int K, bool CK>
+__global__ void __launch_bounds__(SD_THREADS) singular_batch_duffy(const BatchDev *__restrict__ probs, int nprob,
+                                                                   SingBatchTables list, DuffyRule d) {
+    constexpr int GROUPS = SD_THREADS / 8;
+    __shared__ DuffyTable tab;
+    __shared__ double2 scratch[GROUPS][duffy_sums<SD_DP0>()];
+    for (int i = threadIdx.x; i < SD_TAB; i += SD_THREADS) duffy_entry(d, i, tab);
+    __syncthreads();
+    const int group = threadIdx.x / 8;
+    for (int64_t base = (int64_t)blockIdx.x * GROUPS; base < list.npairs; base += (int64_t)gridDim.x * GROUPS) {
+        const int64_t k = base + group;
+        bool valid = k < list.npairs;
+        DuffyTarget tgt = {};
+        int64_t t = 0, s = 0, toff = 0, soff = 0;
+        int npts = 0, cls = 2;
+        if (valid) {
+            const BatchDev &P = probs[find_problem(probs, nprob, k, true)];
+            tgt.g = P.prm.tg;
+            tgt.ne = P.prm.tne;
+            for (int i = 0; i < 4; ++i) tgt.p[i] = P.prm.p[i];
+            tgt.is_complex = true;
+            tgt.dense = P.prm.result;
+            tgt.ld = P.prm.ld;
+            tgt.diag_shift = P.diag_shift;
+            tgt.mirror = true;
+            cls = P.sing_class;
+            t = list.te[k];
+            s = list.se[k];
+            toff = list.toff[k];
+            soff = list.soff[k];
+            npts = (int)list.npts[k];
+            valid = t < tgt.ne && s < tgt.ne && duffy_known(npts, toff, soff);
+        }
+        cls = __reduce_min_sync(0xffffffffu, cls);
+        const auto run = [&](auto c) {
+            duffy_group<BEMPPCUDA_ASM_SCALAR, K, 1, decltype(c)::value, CK, 8>(tgt, tab, d, scratch[group], k, t, s,
+                                                                               toff, soff, npts, valid);
+        };
+        if (cls == 2)
+            run(std::integral_constant<int, 2>());
+        else if (cls == 1)
+            run(std::integral_constant<int, 1>());
+        else
+            run(std::integral_constant<int, 0>());
+        __syncwarp();  // the sums have been read
+    }
+}
+
+template <int K>
+static cudaError_t launch_batch_duffy(const bemppcuda_batch_args *a, const BatchDev *probs, const SingBatchTables &tab,
+                                      cudaStream_t st) {
+    static const DuffyRule rule = duffy_rule4();
+    bool ck = false;
+    for (int i = 0; i < a->nproblems; ++i) ck = ck || a->problems[i].params[1] != 0.0;
+    const int64_t groups = SD_THREADS / 8;
+    const unsigned blocks = (unsigned)std::min<int64_t>((a->npairs + groups - 1) / groups, 16 * (int64_t)bc_sm_count());
+    if (ck)
+        singular_batch_duffy<K, true><<<blocks, SD_THREADS, 0, st>>>(probs, a->nproblems, tab, rule);
+    else
+        singular_batch_duffy<K, false><<<blocks, SD_THREADS, 0, st>>>(probs, a->nproblems, tab, rule);
+    return cudaGetLastError();
+}
+
 static int rows_of(const bemppcuda_batch_args *a) {
     return (a->rows_per_item >= 1 && a->rows_per_item <= DP0_TCHUNK) ? a->rows_per_item : DP0_TCHUNK;
 }
@@ -312,6 +383,7 @@ extern "C" int bemppcuda_batch_prepare(const bemppcuda_batch_args *a, void *stre
         const double theta = fabs(p.params[0]) * p.phase_radius;
         d.phase_class = p.phase_radius > 0.0 ? (theta <= 0.5 ? 2 : (theta <= 1.0 ? 1 : 0)) : 0;
         d.ck = p.params[1] != 0.0;
+        d.sing_class = offset_class64(fmax(fabs(p.params[0]), fabs(p.params[1])) * p.phase_radius);
         d.diag_shift = a->diag_shift;
     }
     char *ws = static_cast<char *>(a->workspace);
@@ -328,7 +400,7 @@ extern "C" int bemppcuda_batch_prepare(const bemppcuda_batch_args *a, void *stre
 
 template <int K>
 static cudaError_t launch_batch(const bemppcuda_batch_args *a, const BatchDev *probs, unsigned long long *counter,
-                                int64_t total_tiles, const QuadRule &rule, int blocks, cudaStream_t st) {
+                                int64_t total_tiles, const QuadRule &rule, int order, int blocks, cudaStream_t st) {
     regular_batch<K><<<blocks, DP0_THREADS, 0, st>>>(probs, a->nproblems, total_tiles, counter, rule);
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess || a->npairs == 0) return err;
@@ -343,12 +415,13 @@ static cudaError_t launch_batch(const bemppcuda_batch_args *a, const BatchDev *p
     tab.woff = a->weights_offsets;
     tab.npts = a->npoints;
     tab.npairs = a->npairs;
+    if (order == SD_Q) return launch_batch_duffy<K>(a, probs, tab, st);
     const unsigned sblocks = (unsigned)((a->npairs + SB_WARPS - 1) / SB_WARPS);
     singular_batch<K><<<sblocks, 32 * SB_WARPS, 0, st>>>(probs, a->nproblems, tab);
     return cudaGetLastError();
 }
 
-extern "C" int bemppcuda_batch_launch(const bemppcuda_batch_args *a, void *stream) {
+static int batch_launch(const bemppcuda_batch_args *a, int order, void *stream) {
     int rc = batch_check(a);
     if (rc) return rc;
     int dev = 0, sms = 0;
@@ -371,13 +444,19 @@ extern "C" int bemppcuda_batch_launch(const bemppcuda_batch_args *a, void *strea
     cudaError_t err = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (err == cudaSuccess) {
         if (a->kernel == BEMPPCUDA_HELMHOLTZ_SLP)
-            err = launch_batch<BEMPPCUDA_HELMHOLTZ_SLP>(a, probs, counter, total_tiles, rule, blocks, st);
+            err = launch_batch<BEMPPCUDA_HELMHOLTZ_SLP>(a, probs, counter, total_tiles, rule, order, blocks, st);
         else
-            err = launch_batch<BEMPPCUDA_HELMHOLTZ_COMBINED>(a, probs, counter, total_tiles, rule, blocks, st);
+            err = launch_batch<BEMPPCUDA_HELMHOLTZ_COMBINED>(a, probs, counter, total_tiles, rule, order, blocks, st);
     }
     if (err != cudaSuccess) {
         bc_set_error("batch_launch: %s", cudaGetErrorString(err));
         return BEMPPCUDA_ERR_CUDA;
     }
     return BEMPPCUDA_OK;
+}
+
+extern "C" int bemppcuda_batch_launch(const bemppcuda_batch_args *a, void *stream) { return batch_launch(a, 0, stream); }
+
+extern "C" int bemppcuda_batch_launch_duffy(const bemppcuda_batch_args *a, int32_t order, void *stream) {
+    return batch_launch(a, (int)order, stream);
 }

@@ -10,6 +10,7 @@
 int bc_regular_launch(const bemppcuda_regular_args *a, cudaStream_t st);
 int bc_apply_launch(const bemppcuda_regular_args *a, const void *x, void *y, cudaStream_t st);
 int bc_singular_launch(const bemppcuda_singular_args *a, cudaStream_t st);
+int bc_singular_duffy_launch(const bemppcuda_singular_args *a, int order, cudaStream_t st);
 int bc_potential_launch(const bemppcuda_potential_args *a, double *workspace, cudaStream_t st);
 int64_t bc_potential_workspace_doubles(int64_t nsupport, int nq);
 
@@ -250,7 +251,8 @@ int bemppcuda_apply_regular(const bemppcuda_regular_args *a, const void *x, void
     return bc_apply_launch(a, x, y, (cudaStream_t)stream);
 }
 
-int bemppcuda_assemble_singular(const bemppcuda_singular_args *a, void *stream) {
+// Shared checks of the two singular entry points.
+static int check_singular(const bemppcuda_singular_args *a) {
     if (!a) {
         bc_set_error("null argument struct");
         return BEMPPCUDA_ERR_INVALID;
@@ -273,7 +275,17 @@ int bemppcuda_assemble_singular(const bemppcuda_singular_args *a, void *stream) 
         bc_set_error("dense ld smaller than the column count");
         return BEMPPCUDA_ERR_INVALID;
     }
-    return bc_singular_launch(a, (cudaStream_t)stream);
+    return BEMPPCUDA_OK;
+}
+
+int bemppcuda_assemble_singular(const bemppcuda_singular_args *a, void *stream) {
+    const int rc = check_singular(a);
+    return rc ? rc : bc_singular_launch(a, (cudaStream_t)stream);
+}
+
+int bemppcuda_assemble_singular_duffy(const bemppcuda_singular_args *a, int32_t order, void *stream) {
+    const int rc = check_singular(a);
+    return rc ? rc : bc_singular_duffy_launch(a, (int)order, (cudaStream_t)stream);
 }
 
 int64_t bemppcuda_potential_workspace_bytes(const bemppcuda_potential_args *a) {

@@ -325,6 +325,16 @@ int bemppcuda_grid_geometry(const double *vertices, int64_t nvertices, const int
 int bemppcuda_assemble_regular(const bemppcuda_regular_args *args, void *stream);
 int bemppcuda_assemble_singular(const bemppcuda_singular_args *args, void *stream);
 
+/* The same for pair lists whose tables are the Sauter-Schwab rules with `order` Gauss points per direction in
+   the layout of SingularPairs (quadrature.py; singular_assembler.py:69-448): coincident rule, six
+   edge remaps (0,1) (1,0) (1,2) (2,1) (0,2) (2,0), three vertex remaps.  Order 4 evaluates the rules
+   from their structure and reads only the elements, offsets and point counts of the pairs (others are
+   skipped when they name no table of that layout); other orders, and spaces with one and three shape
+   functions, go to bemppcuda_assemble_singular.  mirror_weights_offset > 0: every pair is listed in both
+   orders and both spaces are the same, the vertex-adjacent pair t < s then adds both entries (any
+   kernel; the Maxwell fields need equal dof maps only). */
+int bemppcuda_assemble_singular_duffy(const bemppcuda_singular_args *args, int32_t order, void *stream);
+
 /* Matrix-free FP64 apply of the regular part: y += A_reg x, complex128 vectors (x: trial.nsupport
    entries, y: test.nsupport), A_reg the Galerkin matrix of the non-adjacent element pairs evaluated on
    the fly (never stored).  Adjacent pairs and the diagonal contribute nothing here: they are the
@@ -388,6 +398,9 @@ int bemppcuda_batch_prepare(const bemppcuda_batch_args *args, void *stream);
    (a memset and two launches), so it can be captured in a CUDA graph once
    bemppcuda_batch_prepare has run. */
 int bemppcuda_batch_launch(const bemppcuda_batch_args *args, void *stream);
+/* The same for pair lists with the tables of bemppcuda_assemble_singular_duffy (every pair in both orders);
+   orders other than 4 are bemppcuda_batch_launch. */
+int bemppcuda_batch_launch_duffy(const bemppcuda_batch_args *args, int32_t order, void *stream);
 
 int bemppcuda_assemble_identity(const bemppcuda_identity_args *args, void *stream);
 
