@@ -28,15 +28,16 @@ __device__ __forceinline__ double warp_sum64(double v) {
 // blockIdx.x = column block of 128 trial elements, blockIdx.y = row chunk of tile_rows test
 // elements; chunks below the block's last column have no pair i < j and exit at once.  Every
 // lane of a warp runs every row step (the shuffles need the whole warp).
-template <int K, int PHC>
-__global__ void __launch_bounds__(DP0_THREADS) regular_dp0_apply64(RegParams prm, QuadRule rule,
+template <int K, int FORM>
+__global__ void __launch_bounds__(DP0_THREADS) regular_dp0_apply64(RegParams prm, QuadRule rule, OrbitConsts oc,
                                                                    const double2 *__restrict__ x, double2 *y,
                                                                    int tile_rows) {
     const int64_t t0 = (int64_t)blockIdx.y * tile_rows;
     if (t0 >= ((int64_t)blockIdx.x + 1) * DP0_THREADS) return;
     __shared__ TestBlock64s sb;
+    __shared__ double park[form_orbit(FORM) ? SYM_PARK : 1];
     const int tcount = (int)min((int64_t)tile_rows, prm.ntest - t0);
-    stage_sym64(prm, rule, t0, tcount, sb);
+    stage_sym64<FORM>(prm, rule, oc, t0, tcount, sb);
     __syncthreads();
 
     const int64_t si = (int64_t)blockIdx.x * DP0_THREADS + threadIdx.x;
@@ -44,7 +45,7 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_dp0_apply64(RegParams prm
     SymTrial64 tr;
     double2 xj = make_double2(0.0, 0.0);
     if (column) {
-        load_trial_sym64<K, PHC>(prm, rule, si, tr);
+        load_trial_sym64<FORM>(prm, rule, si, park, tr);
         xj = x[si];
     }
     double yr = 0.0, yi = 0.0;  // sum over the block's rows i of A_ji x_i (column j = si)
@@ -54,7 +55,7 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_dp0_apply64(RegParams prm
         // row < si: the pairs above the diagonal; adjacent pairs (and i = j) belong to the singular part
         if (column && row < si && !(prm.grids_identical && shares_vertex(sb.v[tt], tr.sv0, tr.sv1, tr.sv2))) {
             double a_re, a_im, b_re, b_im;
-            pair_sym64<K, PHC>(prm, rule, sb, tt, tr, a_re, a_im, b_re, b_im);
+            pair_sym64<K, FORM>(prm, rule, oc, sb, tt, tr, a_re, a_im, b_re, b_im);
             cr = fma(a_re, xj.x, -a_im * xj.y);
             ci = fma(a_re, xj.y, a_im * xj.x);
             const double2 xi = x[row];
@@ -77,26 +78,17 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_dp0_apply64(RegParams prm
 }
 
 template <int K>
-static cudaError_t launch_apply(const RegParams &prm, const QuadRule &rule, int phase_class, const double2 *x,
-                                double2 *y, cudaStream_t st) {
+static cudaError_t launch_apply(const RegParams &prm, const QuadRule &rule, const OrbitConsts &oc, int form,
+                                const double2 *x, double2 *y, cudaStream_t st) {
     const unsigned bx = (unsigned)((prm.ntrial + DP0_THREADS - 1) / DP0_THREADS);
     // rows per tile as in the assembly's symmetric sweep: fewer when 32-row tiles leave the GPU short of work
     int tile_rows = DP0_TCHUNK;
     const int64_t wave = (int64_t)bc_sm_count() * 3;
-    while (tile_rows > 8 && (int64_t)bx * ((prm.ntest + tile_rows - 1) / tile_rows) / 2 < 4 * wave) tile_rows /= 2;
+    while (tile_rows > 1 && (int64_t)bx * ((prm.ntest + tile_rows - 1) / tile_rows) / 2 < 4 * wave) tile_rows /= 2;
     const dim3 grid(bx, (unsigned)((prm.ntest + tile_rows - 1) / tile_rows));
-    if constexpr (!KernelTraits<K>::helm) {
-        regular_dp0_apply64<K, 0><<<grid, DP0_THREADS, 0, st>>>(prm, rule, x, y, tile_rows);
-    } else {
-        if (prm.p[1] != 0.0)
-            regular_dp0_apply64<K, 3><<<grid, DP0_THREADS, 0, st>>>(prm, rule, x, y, tile_rows);
-        else if (phase_class == 2)
-            regular_dp0_apply64<K, 2><<<grid, DP0_THREADS, 0, st>>>(prm, rule, x, y, tile_rows);
-        else if (phase_class == 1)
-            regular_dp0_apply64<K, 1><<<grid, DP0_THREADS, 0, st>>>(prm, rule, x, y, tile_rows);
-        else
-            regular_dp0_apply64<K, 0><<<grid, DP0_THREADS, 0, st>>>(prm, rule, x, y, tile_rows);
-    }
+    with_form<K>(form, [&](auto f) {
+        regular_dp0_apply64<K, decltype(f)::value><<<grid, DP0_THREADS, 0, st>>>(prm, rule, oc, x, y, tile_rows);
+    });
     return cudaGetLastError();
 }
 
@@ -137,19 +129,21 @@ int bc_apply_launch(const bemppcuda_regular_args *a, const void *x, void *y, cud
     if (prm.ntest == 0) return BEMPPCUDA_OK;
     QuadRule rule;
     fill_rule(rule, a->nq, a->quad_points, a->quad_weights);
-    const double theta = fabs(a->params[0]) * a->phase_radius;
-    const int phase_class = a->phase_radius > 0.0 ? (theta <= 0.5 ? 2 : (theta <= 1.0 ? 1 : 0)) : 0;
+    OrbitRule orbit = {};
+    const bool orbits = orbit_rule(rule, orbit);
+    const OrbitConsts oc = orbits ? orbit_consts(orbit) : OrbitConsts{};
+    const int form = sym_form(a->kernel, prm.p, a->phase_radius, orbits, orbit);
     const double2 *xv = reinterpret_cast<const double2 *>(x);
     double2 *yv = reinterpret_cast<double2 *>(y);
     cudaError_t err;
     switch (a->kernel) {
-    case BEMPPCUDA_LAPLACE_SLP: err = launch_apply<BEMPPCUDA_LAPLACE_SLP>(prm, rule, phase_class, xv, yv, st); break;
-    case BEMPPCUDA_LAPLACE_DLP: err = launch_apply<BEMPPCUDA_LAPLACE_DLP>(prm, rule, phase_class, xv, yv, st); break;
-    case BEMPPCUDA_LAPLACE_ADLP: err = launch_apply<BEMPPCUDA_LAPLACE_ADLP>(prm, rule, phase_class, xv, yv, st); break;
-    case BEMPPCUDA_HELMHOLTZ_SLP: err = launch_apply<BEMPPCUDA_HELMHOLTZ_SLP>(prm, rule, phase_class, xv, yv, st); break;
-    case BEMPPCUDA_HELMHOLTZ_DLP: err = launch_apply<BEMPPCUDA_HELMHOLTZ_DLP>(prm, rule, phase_class, xv, yv, st); break;
-    case BEMPPCUDA_HELMHOLTZ_ADLP: err = launch_apply<BEMPPCUDA_HELMHOLTZ_ADLP>(prm, rule, phase_class, xv, yv, st); break;
-    default: err = launch_apply<BEMPPCUDA_HELMHOLTZ_COMBINED>(prm, rule, phase_class, xv, yv, st); break;
+    case BEMPPCUDA_LAPLACE_SLP: err = launch_apply<BEMPPCUDA_LAPLACE_SLP>(prm, rule, oc, form, xv, yv, st); break;
+    case BEMPPCUDA_LAPLACE_DLP: err = launch_apply<BEMPPCUDA_LAPLACE_DLP>(prm, rule, oc, form, xv, yv, st); break;
+    case BEMPPCUDA_LAPLACE_ADLP: err = launch_apply<BEMPPCUDA_LAPLACE_ADLP>(prm, rule, oc, form, xv, yv, st); break;
+    case BEMPPCUDA_HELMHOLTZ_SLP: err = launch_apply<BEMPPCUDA_HELMHOLTZ_SLP>(prm, rule, oc, form, xv, yv, st); break;
+    case BEMPPCUDA_HELMHOLTZ_DLP: err = launch_apply<BEMPPCUDA_HELMHOLTZ_DLP>(prm, rule, oc, form, xv, yv, st); break;
+    case BEMPPCUDA_HELMHOLTZ_ADLP: err = launch_apply<BEMPPCUDA_HELMHOLTZ_ADLP>(prm, rule, oc, form, xv, yv, st); break;
+    default: err = launch_apply<BEMPPCUDA_HELMHOLTZ_COMBINED>(prm, rule, oc, form, xv, yv, st); break;
     }
     if (err != cudaSuccess) {
         bc_set_error("apply_regular: %s", cudaGetErrorString(err));

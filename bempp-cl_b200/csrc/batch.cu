@@ -10,7 +10,6 @@
 #include <cstring>
 
 #include <algorithm>
-#include <type_traits>
 
 #include "dp0_sym.cuh"
 #include "singular_dp0.cuh"
@@ -28,7 +27,9 @@ struct BatchDev {
     int32_t precision;
     int32_t phase_class;
     int32_t ck;
+    int32_t form;        // of the FP64 symmetric sweep (sym_form)
     int32_t sing_class;  // offset class of the touching pairs
+    int32_t orbits;      // the rule of prepare() was the two-orbit one
     double diag_shift;
 };
 
@@ -36,7 +37,10 @@ constexpr size_t kCounterBytes = 256;
 
 union TileShared {
     TestBlock64 b64;
-    TestBlock64s b64s;
+    struct {
+        TestBlock64s b;
+        double park[SYM_PARK];
+    } s64;
     TestBlock32 b32;
     TestBlock32p b32p;
     TestBlock32q b32q;
@@ -70,23 +74,31 @@ __device__ __forceinline__ void run_tile(const BatchDev &P, const QuadRule &rule
     }
 }
 
-// Symmetric sweep of one problem (Re k > 0 on the mixed path; a complex k is phase class 3 of the FP64
+// Symmetric sweep of one problem (Re k > 0 on the mixed path; a complex k has its forms of the FP64
 // tile and the amplitude split of the mixed one): tile (tx, ty) = columns [128 tx, 128 tx + 128) x rows
 // [rows ty, rows ty + rows).
 template <int K>
-__device__ __forceinline__ void run_tile_sym(const BatchDev &P, const QuadRule &rule, int64_t tx, int64_t ty,
-                                             TileShared &sh) {
+__device__ __forceinline__ void run_tile_sym(const BatchDev &P, const QuadRule &rule, const OrbitConsts &oc,
+                                             int orbits, int64_t tx, int64_t ty, TileShared &sh) {
     const int64_t t0 = ty * P.rows;
     const int rows = P.rows;
     if (P.precision == BEMPPCUDA_FP64) {
-        if (KernelTraits<K>::helm && P.ck)
-            regular_dp0_fp64_sym_tile<K, 3>(P.prm, rule, tx, t0, rows, sh.b64s);
-        else if (P.phase_class == 2)
-            regular_dp0_fp64_sym_tile<K, 2>(P.prm, rule, tx, t0, rows, sh.b64s);
-        else if (P.phase_class == 1)
-            regular_dp0_fp64_sym_tile<K, 1>(P.prm, rule, tx, t0, rows, sh.b64s);
-        else
-            regular_dp0_fp64_sym_tile<K, 0>(P.prm, rule, tx, t0, rows, sh.b64s);
+        // a launch whose rule is not the two-orbit one (the problems were prepared with one that is) takes the
+        // unfactored points form
+        switch (orbits == P.orbits ? P.form : P.ck ? SYM_POINTS_CK : SYM_POINTS) {
+#define BC_BATCH_FORM(F)                                                                                    \
+    case F:                                                                                                 \
+        regular_dp0_fp64_sym_tile<K, F>(P.prm, rule, oc, tx, t0, rows, sh.s64.b, sh.s64.park);              \
+        break
+            BC_BATCH_FORM(SYM_POINTS + 2);
+            BC_BATCH_FORM(SYM_POINTS + 1);
+            BC_BATCH_FORM(SYM_ORBIT_CK + 2);
+            BC_BATCH_FORM(SYM_ORBIT_CK + 1);
+            BC_BATCH_FORM(SYM_ORBIT_CK);
+            BC_BATCH_FORM(SYM_POINTS_CK);
+#undef BC_BATCH_FORM
+        default: regular_dp0_fp64_sym_tile<K, SYM_POINTS>(P.prm, rule, oc, tx, t0, rows, sh.s64.b, sh.s64.park); break;
+        }
     } else if constexpr (KernelTraits<K>::helm) {
         if (P.ck) {
             if (P.phase_class == 2)
@@ -139,7 +151,7 @@ template <int K>
 __global__ void __launch_bounds__(DP0_THREADS) regular_batch(const BatchDev *__restrict__ probs, int nprob,
                                                               int64_t total_tiles,
                                                               unsigned long long *__restrict__ counter,
-                                                              QuadRule rule) {
+                                                              QuadRule rule, OrbitConsts oc, int orbits) {
     __shared__ TileShared sh;
     __shared__ long long s_tile;
     while (true) {
@@ -153,7 +165,7 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_batch(const BatchDev *__r
         if (P.sym) {
             int64_t tx, ty;
             sym_coords(P, local, &tx, &ty);
-            run_tile_sym<K>(P, rule, tx, ty, sh);
+            run_tile_sym<K>(P, rule, oc, orbits, tx, ty, sh);
         } else {
             run_tile<K>(P, rule, local % P.tiles_x, local / P.tiles_x, sh);
         }
@@ -353,6 +365,10 @@ static int batch_check(const bemppcuda_batch_args *a) {
 extern "C" int bemppcuda_batch_prepare(const bemppcuda_batch_args *a, void *stream) {
     int rc = batch_check(a);
     if (rc) return rc;
+    QuadRule rule;
+    fill_rule(rule, a->nq, a->quad_points, a->quad_weights);
+    OrbitRule orbit = {};
+    const bool orbits = orbit_rule(rule, orbit);
     BatchDev *host = new BatchDev[a->nproblems];
     int64_t tiles = 0;
     for (int i = 0; i < a->nproblems; ++i) {
@@ -383,6 +399,8 @@ extern "C" int bemppcuda_batch_prepare(const bemppcuda_batch_args *a, void *stre
         const double theta = fabs(p.params[0]) * p.phase_radius;
         d.phase_class = p.phase_radius > 0.0 ? (theta <= 0.5 ? 2 : (theta <= 1.0 ? 1 : 0)) : 0;
         d.ck = p.params[1] != 0.0;
+        d.form = sym_form(a->kernel, r.p, p.phase_radius, orbits, orbit);
+        d.orbits = orbits ? 1 : 0;
         d.sing_class = offset_class64(fmax(fabs(p.params[0]), fabs(p.params[1])) * p.phase_radius);
         d.diag_shift = a->diag_shift;
     }
@@ -401,7 +419,10 @@ extern "C" int bemppcuda_batch_prepare(const bemppcuda_batch_args *a, void *stre
 template <int K>
 static cudaError_t launch_batch(const bemppcuda_batch_args *a, const BatchDev *probs, unsigned long long *counter,
                                 int64_t total_tiles, const QuadRule &rule, int order, int blocks, cudaStream_t st) {
-    regular_batch<K><<<blocks, DP0_THREADS, 0, st>>>(probs, a->nproblems, total_tiles, counter, rule);
+    OrbitRule orbit = {};
+    const bool orbits = orbit_rule(rule, orbit);
+    regular_batch<K><<<blocks, DP0_THREADS, 0, st>>>(probs, a->nproblems, total_tiles, counter, rule,
+                                                     orbits ? orbit_consts(orbit) : OrbitConsts{}, orbits ? 1 : 0);
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess || a->npairs == 0) return err;
     SingBatchTables tab;

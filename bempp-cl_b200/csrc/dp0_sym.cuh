@@ -15,7 +15,10 @@
 // stores of neighbouring rows of the same warp).
 #pragma once
 
+#include <type_traits>
+
 #include "dp0.cuh"
+#include "orbit_pair.cuh"
 
 namespace bc {
 
@@ -34,180 +37,315 @@ struct SymTraits {
     static constexpr bool supported = slp_part || dlp_part;
 };
 
+// Forms of the FP64 sweep.
+//  points: coordinates differenced per point pair, any 6-point rule; a real wavenumber's exp(ikr) factored about the
+//    centroid distance by offset class (fastmath.cuh), a complex one or exp(-w r) reduced per point pair.
+//  orbit: the two-orbit rule (orbit_pair.cuh), where the amplitudes exp(-Im k r) and exp(-w r) are factored too.
+// The orbit form takes fewer FP64 operations in every kernel, but its chains depend on each other more and it
+// runs the FP64 pipe at 73 - 78 % against 82 - 86 %: with the amplitudes' library exponential gone it is
+// 1.25 - 1.6 times faster (n = 16200: combined field k = 4 + 0.4i 28.5 -> 17.5 ms, modified Helmholtz single
+// layer 11.2 -> 8.9 ms), without them between 0.92 (Laplace single layer) and 1.05 of the points form (double layer).
+constexpr int SYM_POINTS = 0, SYM_POINTS_CK = 3, SYM_ORBIT = 4, SYM_ORBIT_CK = 8;
+constexpr bool form_orbit(int form) { return form >= SYM_ORBIT; }
+constexpr bool form_ck(int form) { return form == SYM_POINTS_CK || form >= SYM_ORBIT_CK; }
+constexpr int form_class(int form) { return form == SYM_POINTS_CK ? 0 : form & 3; }
+
+// The form of a problem: params as in RegParams, radius_sum bounds R_t + R_s (0: unknown).
+inline int sym_form(int kernel, const double *params, double radius_sum, bool orbits, const OrbitRule &orbit) {
+    const bool laplace = kernel <= BEMPPCUDA_LAPLACE_ADLP;
+    const bool modhelm = kernel >= BEMPPCUDA_MODHELM_SLP && kernel <= BEMPPCUDA_MODHELM_ADLP;
+    const bool ck = !laplace && !modhelm && params[1] != 0.0;
+    if (laplace) return SYM_POINTS;
+    const double kmax = ck ? fmax(fabs(params[0]), fabs(params[1])) : fabs(params[0]);
+    const int cls = offset_class64(kmax * radius_sum * (orbits ? orbit.rho : 1.0));
+    if (!ck && !modhelm) return SYM_POINTS + cls;
+    // (the orbit form divides by Re k)
+    if (!orbits || params[0] == 0.0) return ck ? SYM_POINTS_CK : SYM_POINTS;
+    return (ck ? SYM_ORBIT_CK : SYM_ORBIT) + cls;
+}
+
+// Calls f with the form as a compile-time constant, one of those that kernel K has.
+template <int K, class F>
+static void with_form(int form, F &&f) {
+    if constexpr (KernelTraits<K>::helm) {
+        switch (form) {
+        case SYM_POINTS + 2: f(std::integral_constant<int, SYM_POINTS + 2>()); return;
+        case SYM_POINTS + 1: f(std::integral_constant<int, SYM_POINTS + 1>()); return;
+        case SYM_POINTS_CK: f(std::integral_constant<int, SYM_POINTS_CK>()); return;
+        case SYM_ORBIT_CK: f(std::integral_constant<int, SYM_ORBIT_CK>()); return;
+        case SYM_ORBIT_CK + 1: f(std::integral_constant<int, SYM_ORBIT_CK + 1>()); return;
+        case SYM_ORBIT_CK + 2: f(std::integral_constant<int, SYM_ORBIT_CK + 2>()); return;
+        default: break;
+        }
+    } else if constexpr (KernelTraits<K>::modhelm) {
+        switch (form) {
+        case SYM_ORBIT: f(std::integral_constant<int, SYM_ORBIT>()); return;
+        case SYM_ORBIT + 1: f(std::integral_constant<int, SYM_ORBIT + 1>()); return;
+        case SYM_ORBIT + 2: f(std::integral_constant<int, SYM_ORBIT + 2>()); return;
+        default: break;
+        }
+    }
+    f(std::integral_constant<int, SYM_POINTS>());
+}
+
+// A test element of the sweep: the orbit form's centroid and vertex offsets, or the six points and the centroid.
+union TestElem64s {
+    OrbitTest o;
+    struct {
+        double x[NQ6][3], c[3];
+    } p;
+};
+
 struct TestBlock64s {
-    double x[DP0_TCHUNK][NQ6][3];
-    double c[DP0_TCHUNK][3];
+    TestElem64s e[DP0_TCHUNK];
     double n[DP0_TCHUNK][3];
     double ie[DP0_TCHUNK];
     int v[DP0_TCHUNK][3];
 };
 
-// FP64.  PHC 0-2 as in regular_dp0_fp64_tile (real wavenumber); PHC 3 is a complex wavenumber
-// k = kr + i ki: exp(i kr r) from the reduced sine / cosine times exp(-ki r) per point pair and
-// (ikr - 1) / r = -(1/r + ki) + i kr in the double layer (no centroid factoring: the amplitude
-// varies over the pair).  G(x, y) = G(y, x) for complex k too, so the sweep is unchanged.
-// Modified Helmholtz (real, w = p[0]): the Laplace sums with exp(-w r) (single layer) and
-// exp(-w r) (1 + w r) (double layers) per point pair.
+// FP64.  A complex wavenumber k = kr + i ki has exp(ikr) = exp(i kr r) exp(-ki r) and
+// (ikr - 1) / r = -(1/r + ki) + i kr in the double layer; G(x, y) = G(y, x) for complex k too, so the sweep
+// is unchanged.  Modified Helmholtz (real, w = p[0]): the Laplace sums with exp(-w r) (single layer) and
+// exp(-w r) (1 + w r) (double layers).
 //
 // The tile is split into three steps shared by the assembly (stores A_ij, A_ji) and the
 // matrix-free apply (accumulates A x): staging the test block, loading a thread's trial
 // element, and the sweep over the 36 point pairs of one element pair.
 
-// Stage test elements t0 .. t0 + tcount - 1 (points, centroids, normals, areas, vertex ids).
-__device__ __forceinline__ void stage_sym64(const RegParams &prm, const QuadRule &rule, int64_t t0, int tcount,
-                                            TestBlock64s &sb) {
+// Stage test elements t0 .. t0 + tcount - 1.
+template <int FORM>
+__device__ __forceinline__ void stage_sym64(const RegParams &prm, const QuadRule &rule, const OrbitConsts &oc,
+                                            int64_t t0, int tcount, TestBlock64s &sb) {
     for (int idx = threadIdx.x; idx < tcount; idx += blockDim.x) {
         const int64_t t = prm.tsup[t0 + idx];
         Geom g;
         load_geom(prm.tg, prm.tne, t, prm.tnm ? (double)prm.tnm[t] : 1.0, g);
-        double c[3];
+        if (form_orbit(FORM)) {
+            stage_orbit(prm.tg, prm.tne, t, g, oc, sb.e[idx].o);
+        } else {
+            for (int p = 0; p < NQ6; ++p) to_global(g, rule.x[p], rule.y[p], sb.e[idx].p.x[p]);
 #pragma unroll
-        for (int d = 0; d < 3; ++d) c[d] = __ldg(prm.tg + (22 + d) * prm.tne + t);
-        for (int p = 0; p < NQ6; ++p) {
-            double x[3];
-            to_global(g, rule.x[p], rule.y[p], x);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) sb.x[idx][p][d] = x[d];
+            for (int d = 0; d < 3; ++d) sb.e[idx].p.c[d] = __ldg(prm.tg + (22 + d) * prm.tne + t);
         }
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             sb.n[idx][d] = g.n[d];
-            sb.c[idx][d] = c[d];
             sb.v[idx][d] = __ldg(prm.tel + 3 * t + d);
         }
         sb.ie[idx] = g.ie;
     }
 }
 
-// One thread's trial element: geometry, vertex ids, centroid (phase classes 1, 2) and points.
+// One thread's trial element: vertex ids, and the parked orbit fields, or its geometry and points.
 struct SymTrial64 {
-    Geom gs;
     int sv0, sv1, sv2;
-    double sc[3];
-    double y[NQ6][3];
+    OrbitTrial<DP0_THREADS> o;
+    Geom gs;
+    double y[NQ6][3], sc[3];
 };
+constexpr int SYM_PARK = OT_FIELDS * DP0_THREADS;  // doubles of shared memory
 
-template <int K, int PHC>
-__device__ __forceinline__ void load_trial_sym64(const RegParams &prm, const QuadRule &rule, int64_t si,
+template <int FORM>
+__device__ __forceinline__ void load_trial_sym64(const RegParams &prm, const QuadRule &rule, int64_t si, double *park,
                                                  SymTrial64 &tr) {
-    constexpr bool PH = (PHC == 1 || PHC == 2) && SymTraits<K>::helm;
     const int64_t s = prm.ssup[si];
     load_geom(prm.sg, prm.sne, s, prm.snm ? (double)prm.snm[s] : 1.0, tr.gs);
     tr.sv0 = __ldg(prm.sel + 3 * s);
     tr.sv1 = __ldg(prm.sel + 3 * s + 1);
     tr.sv2 = __ldg(prm.sel + 3 * s + 2);
+    if (form_orbit(FORM)) {
+        tr.o = park_orbit_trial<DP0_THREADS>(prm.sg, prm.sne, s, tr.gs, park);
+    } else {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) tr.sc[d] = PH ? __ldg(prm.sg + (22 + d) * prm.sne + s) : 0.0;
+        for (int q = 0; q < NQ6; ++q) to_global(tr.gs, rule.x[q], rule.y[q], tr.y[q]);
 #pragma unroll
-    for (int q = 0; q < NQ6; ++q) to_global(tr.gs, rule.x[q], rule.y[q], tr.y[q]);
+        for (int d = 0; d < 3; ++d) tr.sc[d] = form_class(FORM) > 0 ? __ldg(prm.sg + (22 + d) * prm.sne + s) : 0.0;
+    }
+}
+
+// The sums of a pair: s single layer, u double layer with the trial normal, v with the test normal
+// (weights included, 1 / (4 pi), areas and the factor at r_c left out; u and v as -u_re + i u_im).
+struct SymSums {
+    double s_re, s_im, u_re, u_im, v_re, v_im;
+};
+
+// One test point's terms of the six trial points; yw[q] = (x - y_q) . n_t, xn = (y - x) . n_s.
+template <int K, int FORM>
+__device__ __forceinline__ void point_sym64(const double r2[6], const double w[6], double wp, double xn,
+                                            const double yw[6], double kr, double ki, double krc, double kirc,
+                                            SymSums &a) {
+    using ST = SymTraits<K>;
+    constexpr bool CK = form_ck(FORM) && ST::helm;
+    constexpr int CLS = form_class(FORM);
+    double pr = 0.0, pi = 0.0, ur = 0.0, ui = 0.0, vr = 0.0, vi = 0.0;
+    const double ik = ST::helm && form_orbit(FORM) ? 1.0 / kr : 0.0;
+#pragma unroll
+    for (int q = 0; q < NQ6; ++q) {
+        const double rinv = rsqrt64(r2[q]);
+        double f = w[q] * rinv;
+        if (!ST::helm) {
+            double e = 1.0, e1 = 1.0;  // modified Helmholtz: exp(-w r), exp(-w r) (1 + w r)
+            if (ST::modhelm) {
+                const double r = r2[q] * rinv;
+                e = exp_off64<CLS>(fma(-kr, r, krc));
+                e1 = e * fma(kr, r, 1.0);
+            }
+            if (ST::slp_part) pr = ST::modhelm ? fma(f, e, pr) : pr + f;
+            if (ST::dlp_part) {
+                const double g3 = ST::modhelm ? f * rinv * rinv * e1 : f * rinv * rinv;
+                ur += g3;
+                vr = fma(g3, yw[q], vr);
+            }
+        } else {
+            const double r = r2[q] * rinv;
+            double sn, cs;
+            sincos_off64<CLS>(fma(kr, r, -krc), &sn, &cs);
+            if (CK) f *= exp_off64<CLS>(fma(-ki, r, kirc));
+            if (ST::slp_part) {
+                pr = fma(f, cs, pr);
+                pi = fma(f, sn, pi);
+            }
+            if (ST::dlp_part) {
+                // (ikr - 1) e^{ikr} / r^3 is -h1 + i h2 per unit f (dot) / r; the orbit forms carry h / kr
+                const double fr = f * rinv, rk = CK ? rinv + ki : rinv;
+                double h1, h2;
+                if (form_orbit(FORM)) {
+                    const double rho = rk * ik;
+                    h1 = fma(rho, cs, sn);
+                    h2 = fma(-rho, sn, cs);
+                } else {
+                    h1 = fma(rk, cs, kr * sn);
+                    h2 = fma(kr, cs, -rk * sn);
+                }
+                const double gt = fr * yw[q];
+                ur = fma(fr, h1, ur);
+                ui = fma(fr, h2, ui);
+                vr = fma(gt, h1, vr);
+                vi = fma(gt, h2, vi);
+            }
+        }
+    }
+    const double wn = wp * xn;
+    a.s_re = fma(wp, pr, a.s_re);
+    a.s_im = fma(wp, pi, a.s_im);
+    a.u_re = fma(wn, ur, a.u_re);
+    a.u_im = fma(wn, ui, a.u_im);
+    a.v_re = fma(wp, vr, a.v_re);
+    a.v_im = fma(wp, vi, a.v_im);
+}
+
+// The sums of an element pair in the orbit form (NEAR: differenced coordinates, orbit_r2).
+template <int K, int FORM, bool NEAR>
+__device__ __forceinline__ void sums_sym64(const OrbitTest &te, const OrbitTrial<DP0_THREADS> &tr, const OrbitPair &p,
+                                           const OrbitConsts &oc, double Dn, const double yw[6], double kr, double ki,
+                                           SymSums &a) {
+    using ST = SymTraits<K>;
+    const double w[6] = {oc.w[0], oc.w[0], oc.w[0], oc.w[1], oc.w[1], oc.w[1]};
+#pragma unroll 1
+    for (int i = 0; i < 3; ++i) {
+        const double e[3] = {te.e[i][0], te.e[i][1], te.e[i][2]};
+        double f0[3], f1[3], en = 0.0;
+        tr.f(f0, f1);
+        const double De = odot(p.D, e), E0 = odot(e, f0), E1 = odot(e, f1);
+        const double E[3] = {E0, E1, -(E0 + E1)};
+        if (ST::dlp_part) {
+            double sn[3];
+            tr.n(sn);
+            en = odot(e, sn);
+        }
+#pragma unroll 1
+        for (int op = 0; op < 2; ++op) {
+            double r2[6];
+            orbit_r2<NEAR>(p, tr, oc, op, e, te.ge[op][i], De, E, r2);
+            point_sym64<K, FORM>(r2, w, oc.w[op], fma(-oc.g[op], en, Dn), yw, kr, ki, p.krc, p.kirc, a);
+        }
+    }
 }
 
 // A_ij and A_ji of the non-adjacent pair (test element tt of the block, the thread's trial element).
-template <int K, int PHC>
-__device__ __forceinline__ void pair_sym64(const RegParams &prm, const QuadRule &rule, const TestBlock64s &sb,
-                                           int tt, const SymTrial64 &tr, double &a_re, double &a_im, double &b_re,
-                                           double &b_im) {
+template <int K, int FORM>
+__device__ __forceinline__ void pair_sym64(const RegParams &prm, const QuadRule &rule, const OrbitConsts &oc,
+                                           const TestBlock64s &sb, int tt, const SymTrial64 &tr, double &a_re,
+                                           double &a_im, double &b_re, double &b_im) {
     using ST = SymTraits<K>;
-    constexpr bool PH = (PHC == 1 || PHC == 2) && ST::helm;
-    constexpr bool CK = PHC == 3 && ST::helm;
-    const Geom &gs = tr.gs;
+    constexpr bool ORB = form_orbit(FORM), CK = form_ck(FORM) && ST::helm;
+    constexpr int CLS = form_class(FORM), FAM = kernel_family<K>();
     const double kr = prm.p[0], ki = CK ? prm.p[1] : 0.0, etar = prm.p[2], etai = prm.p[3];
-    double rc = 0.0, ph_s = 0.0, ph_c = 1.0;
-    if (PH) {
-        const double D0 = tr.sc[0] - sb.c[tt][0], D1 = tr.sc[1] - sb.c[tt][1], D2 = tr.sc[2] - sb.c[tt][2];
-        rc = sqrt(fma(D2, D2, fma(D1, D1, D0 * D0)));
-        sincos_cw64(kr * rc, &ph_s, &ph_c);
-    }
-    // Normal terms: (y - x).n_j = (v0_j - x).n_j since y lies in the plane of j (one value per
-    // test point, applied after the sum over q), and (x - y).n_i = (c_i - y).n_i since x lies in
-    // the plane of i (one value per trial point)
-    double ynt[NQ6];
-    if (ST::dlp_part)
+    const double tn[3] = {sb.n[tt][0], sb.n[tt][1], sb.n[tt][2]};
+    // Normal terms: (y - x).n_s is one value per test point since y lies in the plane of the trial element,
+    // (x - y).n_t one value per trial point since x lies in the plane of the test element
+    double yw[NQ6];
+    SymSums a = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    double ph_c = 1.0, ph_s = 0.0;
+    if constexpr (ORB) {
+        const OrbitTest &te = sb.e[tt].o;
+        OrbitPair p;
+        orbit_pair<FAM, CK, CLS>(te, tr.o, oc, kr, ki, p);
+        double Dn = 0.0;
+        if (ST::dlp_part) {
+            double sn[3], v0[3], v1[3];
+            tr.o.n(sn);
+            tr.o.f(v0, v1);
+            Dn = odot(p.D, sn);
+            const double Dt = odot(p.D, tn), f0 = odot(v0, tn), f1 = odot(v1, tn);
+            const double f[3] = {f0, f1, -(f0 + f1)};
 #pragma unroll
-        for (int q = 0; q < NQ6; ++q)
-            ynt[q] = fma(sb.c[tt][2] - tr.y[q][2], sb.n[tt][2],
-                         fma(sb.c[tt][1] - tr.y[q][1], sb.n[tt][1], (sb.c[tt][0] - tr.y[q][0]) * sb.n[tt][0]));
-    double s0r = 0.0, s0i = 0.0, u_re = 0.0, u_im = 0.0, v_re = 0.0, v_im = 0.0;
-    for (int p = 0; p < NQ6; ++p) {
-        const double x0 = sb.x[tt][p][0], x1 = sb.x[tt][p][1], x2 = sb.x[tt][p][2];
-        double xn = 0.0;
-        if (ST::dlp_part)
-            xn = fma(gs.v0[2] - x2, gs.n[2], fma(gs.v0[1] - x1, gs.n[1], (gs.v0[0] - x0) * gs.n[0]));
-        double pr = 0.0, pi = 0.0, ur = 0.0, ui = 0.0, vr = 0.0, vi = 0.0;
-#pragma unroll
-        for (int q = 0; q < NQ6; ++q) {
-            const double d0 = tr.y[q][0] - x0, d1 = tr.y[q][1] - x1, d2 = tr.y[q][2] - x2;
-            const double r2 = fma(d2, d2, fma(d1, d1, d0 * d0));
-            const double rinv = rsqrt64(r2);
-            const double f = rule.w[q] * rinv;
-            if (!ST::helm) {
-                double e = 1.0, e1 = 1.0;  // modified Helmholtz: exp(-w r), exp(-w r) (1 + w r)
-                if (ST::modhelm) {
-                    const double r = r2 * rinv;
-                    e = exp(-kr * r);
-                    e1 = e * fma(kr, r, 1.0);
-                }
-                if (ST::slp_part) pr = ST::modhelm ? fma(f, e, pr) : pr + f;
-                if (ST::dlp_part) {
-                    const double g3 = ST::modhelm ? f * rinv * rinv * e1 : f * rinv * rinv;
-                    ur += g3;
-                    vr = fma(g3, ynt[q], vr);
-                }
-            } else {
-                const double r = r2 * rinv;
-                double sn, cs;
-                if (PH && PHC == 2)
-                    sincos_half64(kr * (r - rc), &sn, &cs);
-                else if (PH)
-                    sincos_small64(kr * (r - rc), &sn, &cs);
-                else
-                    sincos_cw64(kr * r, &sn, &cs);
-                if (CK) {
-                    const double am = exp(-ki * r);
-                    sn *= am;
-                    cs *= am;
-                }
-                if (ST::slp_part) {
-                    pr = fma(f, cs, pr);
-                    pi = fma(f, sn, pi);
-                }
-                if (ST::dlp_part) {
-                    // (ikr - 1) e^{ikr} / r^3: -h1 + i h2 per unit f (dot) / r
-                    const double fr = f * rinv, rk = CK ? rinv + ki : rinv;
-                    const double h1 = fma(rk, cs, kr * sn), h2 = fma(kr, cs, -rk * sn);
-                    const double gt = fr * ynt[q];
-                    ur = fma(fr, h1, ur);
-                    ui = fma(fr, h2, ui);
-                    vr = fma(gt, h1, vr);
-                    vi = fma(gt, h2, vi);
-                }
-            }
+            for (int q = 0; q < NQ6; ++q) yw[q] = -fma(oc.g[q / 3], f[q % 3], Dt);
         }
-        const double wp = rule.w[p], wpn = wp * xn;
-        s0r = fma(wp, pr, s0r);
-        s0i = fma(wp, pi, s0i);
-        u_re = fma(wpn, ur, u_re);
-        u_im = fma(wpn, ui, u_im);
-        v_re = fma(wp, vr, v_re);
-        v_im = fma(wp, vi, v_im);
+        if (p.far)
+            sums_sym64<K, FORM, false>(te, tr.o, p, oc, Dn, yw, kr, ki, a);
+        else
+            sums_sym64<K, FORM, true>(te, tr.o, p, oc, Dn, yw, kr, ki, a);
+        orbit_phase<FAM, CK, CLS>(p, ph_c, ph_s);
+        if (ST::helm && ST::dlp_part) {  // the sums of h / kr
+            a.u_re *= kr;
+            a.u_im *= kr;
+            a.v_re *= kr;
+            a.v_im *= kr;
+        }
+    } else {
+        const double(*x)[3] = sb.e[tt].p.x, *c = sb.e[tt].p.c;
+        const Geom &gs = tr.gs;
+        double krc = 0.0;
+        if (CLS > 0) {
+            const double D0 = tr.sc[0] - c[0], D1 = tr.sc[1] - c[1], D2 = tr.sc[2] - c[2];
+            krc = kr * sqrt(fma(D2, D2, fma(D1, D1, D0 * D0)));
+            sincos_cw64(krc, &ph_s, &ph_c);
+        }
+        if (ST::dlp_part)
+#pragma unroll
+            for (int q = 0; q < NQ6; ++q)
+                yw[q] = fma(c[2] - tr.y[q][2], tn[2], fma(c[1] - tr.y[q][1], tn[1], (c[0] - tr.y[q][0]) * tn[0]));
+        for (int p = 0; p < NQ6; ++p) {
+            const double x0 = x[p][0], x1 = x[p][1], x2 = x[p][2];
+            double xn = 0.0, r2[6];
+            if (ST::dlp_part)
+                xn = fma(gs.v0[2] - x2, gs.n[2], fma(gs.v0[1] - x1, gs.n[1], (gs.v0[0] - x0) * gs.n[0]));
+#pragma unroll
+            for (int q = 0; q < NQ6; ++q) {
+                const double d0 = tr.y[q][0] - x0, d1 = tr.y[q][1] - x1, d2 = tr.y[q][2] - x2;
+                r2[q] = fma(d2, d2, fma(d1, d1, d0 * d0));
+            }
+            point_sym64<K, FORM>(r2, rule.w, rule.w[p], xn, yw, kr, ki, krc, 0.0, a);
+        }
     }
     // kernel values: Laplace DLP -sum f dot / r^2; Helmholtz DLP -u_re + i u_im
     double dr = 0.0, di = 0.0, er = 0.0, ei = 0.0;  // double-layer parts of A_ij, A_ji
     if (ST::dlp_part) {
-        dr = -u_re;
-        di = ST::helm ? u_im : 0.0;
-        er = -v_re;
-        ei = ST::helm ? v_im : 0.0;
+        dr = -a.u_re;
+        di = ST::helm ? a.u_im : 0.0;
+        er = -a.v_re;
+        ei = ST::helm ? a.v_im : 0.0;
     }
     if (K == BEMPPCUDA_HELMHOLTZ_COMBINED) {
-        const double sr = fma(etar, s0r, -etai * s0i), sim = fma(etar, s0i, etai * s0r);
+        const double sr = fma(etar, a.s_re, -etai * a.s_im), sim = fma(etar, a.s_im, etai * a.s_re);
         a_re = dr + sr;
         a_im = di + sim;
         b_re = er + sr;
         b_im = ei + sim;
     } else if (ST::slp_part) {
-        a_re = b_re = s0r;
-        a_im = b_im = s0i;
+        a_re = b_re = a.s_re;
+        a_im = b_im = a.s_im;
     } else if (ST::swap) {
         a_re = er;
         a_im = ei;
@@ -219,39 +357,43 @@ __device__ __forceinline__ void pair_sym64(const RegParams &prm, const QuadRule 
         b_re = er;
         b_im = ei;
     }
-    const double scale = BC_INV_4PI * sb.ie[tt] * gs.ie;
-    if (PH) {
-        double t = a_re * ph_c - a_im * ph_s;
-        a_im = (a_re * ph_s + a_im * ph_c) * scale;
-        a_re = t * scale;
-        t = b_re * ph_c - b_im * ph_s;
-        b_im = (b_re * ph_s + b_im * ph_c) * scale;
-        b_re = t * scale;
+    const double scale = BC_INV_4PI * sb.ie[tt] * (ORB ? tr.o.ld(OT_IE) : tr.gs.ie);
+    ph_c *= scale;
+    if (CLS > 0 && ST::helm) {
+        ph_s *= scale;
+        double t = fma(a_re, ph_c, -a_im * ph_s);
+        a_im = fma(a_re, ph_s, a_im * ph_c);
+        a_re = t;
+        t = fma(b_re, ph_c, -b_im * ph_s);
+        b_im = fma(b_re, ph_s, b_im * ph_c);
+        b_re = t;
     } else {
-        a_re *= scale;
-        a_im *= scale;
-        b_re *= scale;
-        b_im *= scale;
+        a_re *= ph_c;
+        a_im *= ph_c;
+        b_re *= ph_c;
+        b_im *= ph_c;
     }
 }
 
-template <int K, int PHC, bool STRIPE = false>
+template <int K, int FORM, bool STRIPE = false>
 __device__ __forceinline__ void regular_dp0_fp64_sym_tile(const RegParams &prm, const QuadRule &rule,
-                                                        int64_t tile_x, int64_t t0, int rows, TestBlock64s &sb) {
+                                                        const OrbitConsts &oc, int64_t tile_x, int64_t t0, int rows,
+                                                        TestBlock64s &sb, double *park) {
     const int tcount = (int)min((int64_t)rows, prm.ntest - t0);
-    stage_sym64(prm, rule, t0, tcount, sb);
+    stage_sym64<FORM>(prm, rule, oc, t0, tcount, sb);
     __syncthreads();
 
     const int64_t si = tile_x * DP0_THREADS + threadIdx.x;
     if (si < prm.ntrial && t0 <= si) {
         SymTrial64 tr;
-        load_trial_sym64<K, PHC>(prm, rule, si, tr);
+        load_trial_sym64<FORM>(prm, rule, si, park, tr);
+#pragma unroll 1
         for (int tt = 0; tt < tcount; ++tt) {
             const int64_t row = t0 + tt;
             if (row > si) break;  // rows increase with tt: the rest of this column lies below the diagonal
             const bool adj = row == si || (prm.grids_identical && shares_vertex(sb.v[tt], tr.sv0, tr.sv1, tr.sv2));
             double a_re = 0.0, a_im = 0.0, b_re = 0.0, b_im = 0.0;  // A_ij, A_ji
-            if (!adj) pair_sym64<K, PHC>(prm, rule, sb, tt, tr, a_re, a_im, b_re, b_im);
+            if (!adj) pair_sym64<K, FORM>(prm, rule, oc, sb, tt, tr, a_re, a_im, b_re, b_im);
             store_pair<STRIPE>(prm, row, si, adj, a_re, a_im, b_re, b_im);
         }
     }

@@ -5,7 +5,7 @@
 // hypersingular_regular (:1078-1467), maxwell_efield_regular_assembler
 // (:1853-1970) and maxwell_mfield_regular_assembler (:2151-2278).
 //
-// Two kernels:
+// Kernels:
 //  * regular_dp0<K, MIXED>: piecewise-constant test and trial spaces with the
 //    identity dof map, 6-point rule.  One thread owns one trial element
 //    (a matrix column) and sweeps a block of test elements (rows) staged in
@@ -16,20 +16,20 @@
 //    per point only the offset r - r_c = (2 D.e + e.e) / (r + r_c) enters
 //    the FP32 phase, so the phase error stays ~1e-7 rad independently of
 //    k r.  The 6-point inner sums are FP32, the per-entry sum is FP64.
-//  * regular_p1<ASM, K, ...> (p1.cuh): scalar and hypersingular operators on
-//    P1 / DP1 / P0 spaces, 6-point rule, real wavenumber.
-//  * regular_rwg<ASM, ...> (rwg.cuh): Maxwell electric / magnetic field on
-//    RWG / SNC spaces, 6-point rule, real nonzero wavenumber.
+//  * regular_p1_points (p1_points.cuh) and regular_p1 (p1.cuh): scalar and
+//    hypersingular operators on P1 / DP1 / P0 spaces, 6-point rule
+//    (two-orbit in the latter).
+//  * regular_rwg_points, regular_rwg_orbit (rwg.cuh): Maxwell electric /
+//    magnetic field on RWG / SNC spaces, 6-point rule, nonzero wavenumber, real
+//    (any rule) or complex (two-orbit).
 //  * regular_generic<ASM, K>: every other scalar / hypersingular / Maxwell
 //    assembly with 1 or 3 shape functions and any rule (<= 16 points).  One
 //    thread per element pair; the local nshape x nshape block is scattered
 //    with atomicAdd into the (pre-zeroed or accumulating) result.
 #include <cstdio>
 
-#include "dp0_sym.cuh"
-#include "p1.cuh"
-#include "p1_mixed.cuh"
-#include "rwg.cuh"
+#include "dp0_sym.cuh"  // sym_form
+#include "regular.cuh"
 
 namespace bc {
 
@@ -233,231 +233,6 @@ __global__ void __launch_bounds__(GEN_THREADS) regular_generic(RegParams prm, Qu
     }
 }
 
-// Symmetric sweeps: blockIdx.x = column block, blockIdx.y = row chunk; chunks
-// that start below the block's last column have no pair i <= j and exit
-// before touching shared memory.
-template <int K, int PHC, bool STRIPE = false>
-__global__ void __launch_bounds__(DP0_THREADS) regular_dp0_fp64_sym(RegParams prm, QuadRule rule, int64_t row0,
-                                                                    int64_t row1, int tile_rows) {
-    const int64_t t0 = row0 + (int64_t)blockIdx.y * tile_rows;
-    if (t0 >= ((int64_t)blockIdx.x + 1) * DP0_THREADS) return;
-    __shared__ TestBlock64s sb;
-    regular_dp0_fp64_sym_tile<K, PHC, STRIPE>(prm, rule, blockIdx.x, t0, (int)min((int64_t)tile_rows, row1 - t0),
-                                              sb);
-}
-
-// CTAs per SM the mixed symmetric sweep is compiled for (register cap 170 at
-// 3): timed at L6, 3 and 4 are equal, 2 is 10 % slower.
-#ifndef BC_MSYM_MIN_BLOCKS
-#define BC_MSYM_MIN_BLOCKS 3
-#endif
-
-template <int K, int PHC, bool STRIPE = false, bool CK = false>
-__global__ void __launch_bounds__(DP0_THREADS, BC_MSYM_MIN_BLOCKS) regular_dp0_mixed_sym(RegParams prm, QuadRule rule,
-                                                                                      int64_t row0, int64_t row1,
-                                                                                      int tile_rows) {
-    const int64_t t0 = row0 + (int64_t)blockIdx.y * tile_rows;
-    if (t0 >= ((int64_t)blockIdx.x + 1) * DP0_THREADS) return;
-    __shared__ TestBlock32q sb;
-    regular_dp0_mixed_sym_tile<K, PHC, STRIPE, CK>(prm, rule, blockIdx.x, t0,
-                                                   (int)min((int64_t)tile_rows, row1 - t0), sb);
-}
-
-// The mixed symmetric sweep in its phase class, real or (Helmholtz) complex wavenumber.
-template <int K, bool STRIPE, bool CK>
-static void mixed_sym_phase(const RegParams &prm, const QuadRule &rule, int phase_class, int64_t row0, int64_t row1,
-                            int tile_rows, dim3 sgrid, cudaStream_t st) {
-    if (phase_class == 2)
-        regular_dp0_mixed_sym<K, 2, STRIPE, CK><<<sgrid, DP0_THREADS, 0, st>>>(prm, rule, row0, row1, tile_rows);
-    else if (phase_class == 1)
-        regular_dp0_mixed_sym<K, 1, STRIPE, CK><<<sgrid, DP0_THREADS, 0, st>>>(prm, rule, row0, row1, tile_rows);
-    else
-        regular_dp0_mixed_sym<K, 0, STRIPE, CK><<<sgrid, DP0_THREADS, 0, st>>>(prm, rule, row0, row1, tile_rows);
-}
-
-template <int K, bool STRIPE>
-static void launch_mixed_sym(const RegParams &prm, const QuadRule &rule, int phase_class, int64_t row0, int64_t row1,
-                             int tile_rows, dim3 sgrid, cudaStream_t st) {
-    if constexpr (KernelTraits<K>::helm) {
-        if (prm.p[1] != 0.0) {
-            mixed_sym_phase<K, STRIPE, true>(prm, rule, phase_class, row0, row1, tile_rows, sgrid, st);
-            return;
-        }
-    }
-    mixed_sym_phase<K, STRIPE, false>(prm, rule, phase_class, row0, row1, tile_rows, sgrid, st);
-}
-
-// Kernels with a stripe-mode instance (the multi-GPU symmetric stripes): the Helmholtz family, the
-// combined field and the Laplace single layer.
-template <int K>
-constexpr bool stripe_kernel() {
-    return K == BEMPPCUDA_HELMHOLTZ_SLP || K == BEMPPCUDA_HELMHOLTZ_DLP || K == BEMPPCUDA_HELMHOLTZ_ADLP ||
-           K == BEMPPCUDA_HELMHOLTZ_COMBINED || K == BEMPPCUDA_LAPLACE_SLP;
-}
-
-// The symmetric sweep of launch_dp0 in stripe mode (real or complex wavenumber; mixed or FP64).
-template <int K>
-static cudaError_t launch_dp0_stripe(const RegParams &prm, const QuadRule &rule, int mixed, int phase_class,
-                                     int64_t row0, int64_t row1, int tile_rows, dim3 sgrid, cudaStream_t st) {
-    if constexpr (stripe_kernel<K>()) {
-        if (mixed) {
-            launch_mixed_sym<K, true>(prm, rule, phase_class, row0, row1, tile_rows, sgrid, st);
-        } else if (!KernelTraits<K>::helm) {
-            regular_dp0_fp64_sym<K, 0, true><<<sgrid, DP0_THREADS, 0, st>>>(prm, rule, row0, row1, tile_rows);
-        } else if (prm.p[1] != 0.0) {
-            regular_dp0_fp64_sym<K, 3, true><<<sgrid, DP0_THREADS, 0, st>>>(prm, rule, row0, row1, tile_rows);
-        } else if (phase_class == 2) {
-            regular_dp0_fp64_sym<K, 2, true><<<sgrid, DP0_THREADS, 0, st>>>(prm, rule, row0, row1, tile_rows);
-        } else if (phase_class == 1) {
-            regular_dp0_fp64_sym<K, 1, true><<<sgrid, DP0_THREADS, 0, st>>>(prm, rule, row0, row1, tile_rows);
-        } else {
-            regular_dp0_fp64_sym<K, 0, true><<<sgrid, DP0_THREADS, 0, st>>>(prm, rule, row0, row1, tile_rows);
-        }
-        return cudaGetLastError();
-    } else {
-        return cudaErrorInvalidValue;
-    }
-}
-
-template <int K>
-static cudaError_t launch_dp0(const RegParams &prm, const QuadRule &rule, int mixed, int phase_class, bool sym,
-                              int64_t row0, int64_t row1, cudaStream_t st) {
-    dim3 grid((unsigned)((prm.ntrial + DP0_THREADS - 1) / DP0_THREADS), (unsigned)((prm.ntest + DP0_TCHUNK - 1) / DP0_TCHUNK));
-    if constexpr (SymTraits<K>::supported) {
-        // same DP0 space on both sides; the mixed tiles need Re k > 0 or omega > 0 (scaled units; a
-        // complex k adds the amplitude split), the FP64 tiles take a complex k as phase class 3
-        const bool helm = KernelTraits<K>::helm;
-        const bool ck_sym = helm && prm.p[1] != 0.0;
-        const bool sweep_ok = helm || KernelTraits<K>::modhelm ? (!mixed || prm.p[0] > 0.0) : true;
-        if (sym && sweep_ok) {
-            // rows per tile: 32, or 16 / 8 when 32-row tiles would leave the GPU under four waves of
-            // working CTAs (about half the tiles lie below the diagonal and exit; 3 CTAs per SM)
-            int tile_rows = DP0_TCHUNK;
-            const int64_t wave = (int64_t)bc_sm_count() * 3;
-            while (tile_rows > 8 && (int64_t)grid.x * ((row1 - row0 + tile_rows - 1) / tile_rows) / 2 < 4 * wave)
-                tile_rows /= 2;
-            const dim3 sgrid(grid.x, (unsigned)((row1 - row0 + tile_rows - 1) / tile_rows));
-            if (prm.tresult) return launch_dp0_stripe<K>(prm, rule, mixed, phase_class, row0, row1, tile_rows, sgrid, st);
-            if (mixed) {
-                launch_mixed_sym<K, false>(prm, rule, phase_class, row0, row1, tile_rows, sgrid, st);
-                return cudaGetLastError();
-            }
-            if constexpr (!KernelTraits<K>::helm) {  // no phase: one instance
-                regular_dp0_fp64_sym<K, 0><<<sgrid, DP0_THREADS, 0, st>>>(prm, rule, row0, row1, tile_rows);
-            } else {
-                if (ck_sym)
-                    regular_dp0_fp64_sym<K, 3><<<sgrid, DP0_THREADS, 0, st>>>(prm, rule, row0, row1, tile_rows);
-                else if (phase_class == 2)
-                    regular_dp0_fp64_sym<K, 2><<<sgrid, DP0_THREADS, 0, st>>>(prm, rule, row0, row1, tile_rows);
-                else if (phase_class == 1)
-                    regular_dp0_fp64_sym<K, 1><<<sgrid, DP0_THREADS, 0, st>>>(prm, rule, row0, row1, tile_rows);
-                else
-                    regular_dp0_fp64_sym<K, 0><<<sgrid, DP0_THREADS, 0, st>>>(prm, rule, row0, row1, tile_rows);
-            }
-            return cudaGetLastError();
-        }
-    }
-    const bool ck = prm.p[1] != 0.0 && KernelTraits<K>::helm;
-    // the packed path measures lengths in units of 1/k: Helmholtz needs k > 0
-    const bool packed = !KernelTraits<K>::helm || prm.p[0] > 0.0;
-    if constexpr (!KernelTraits<K>::modhelm) {
-        if (mixed && !ck && packed) {
-            if (phase_class == 2)
-                regular_dp0_mixed2<K, 2><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-            else if (phase_class == 1)
-                regular_dp0_mixed2<K, 1><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-            else
-                regular_dp0_mixed2<K, 0><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-            return cudaGetLastError();
-        }
-    }
-    if (row0 != 0 || row1 != prm.ntest) return cudaErrorInvalidValue;  // a row range needs the symmetric sweep
-    if (mixed) {
-        if (ck)
-            regular_dp0_mixed<K, true, 0><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else if (phase_class == 2)
-            regular_dp0_mixed<K, false, 2><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else if (phase_class == 1)
-            regular_dp0_mixed<K, false, 1><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else
-            regular_dp0_mixed<K, false, 0><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-    } else {
-        if (ck)
-            regular_dp0_fp64<K, true, 0><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else if (phase_class == 2)
-            regular_dp0_fp64<K, false, 2><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else if (phase_class == 1)
-            regular_dp0_fp64<K, false, 1><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else
-            regular_dp0_fp64<K, false, 0><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-    }
-    return cudaGetLastError();
-}
-
-// Row blocks of the Maxwell sweeps (regular_rwg, regular_p1_mixed on RWG): 32 test elements per
-// CTA, or 16 when 32 would leave the GPU under four waves of working CTAs (a symmetric sweep's CTAs
-// below the diagonal exit at once; 3 CTAs per SM).  The kernels take their chunk height as
-// ceil(ntest / gridDim.y).  L4 (2048 elements), regular pass: electric field 0.52 -> 0.40 ms FP64,
-// 0.39 -> 0.31 ms mixed; magnetic field 0.38 -> 0.35 ms mixed.  The P1 scalar kernels keep 32 rows
-// as a compile-time height: a runtime one made the mixed hypersingular operator 4 % slower at L5.
-static unsigned lin_row_blocks(int64_t ntrial, int64_t ntest, bool sym) {
-    static_assert(P1_TCHUNK == 32 && RWG_TCHUNK == 32, "row blocks of 32 or 16 test elements");
-    const int64_t cols = (ntrial + DP0_THREADS - 1) / DP0_THREADS;
-    const int64_t wave = (int64_t)bc_sm_count() * 3;
-    const int rows = cols * ((ntest + 31) / 32) / (sym ? 2 : 1) < 4 * wave ? 16 : 32;
-    return (unsigned)((ntest + rows - 1) / rows);
-}
-
-template <int ASM, int K, int NT, int NS, bool SYM>
-static void launch_p1_phase(const RegParams &prm, const QuadRule &rule, int phase_class, dim3 grid, cudaStream_t st) {
-    // the phase classes only concern exp(ikr): one instance for Laplace and modified Helmholtz
-    if constexpr (K != BEMPPCUDA_HELMHOLTZ_SLP && K != BEMPPCUDA_HELMHOLTZ_DLP && K != BEMPPCUDA_HELMHOLTZ_ADLP) {
-        regular_p1<ASM, K, NT, NS, 0, SYM><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-    } else {
-        if (phase_class == 3)  // complex wavenumber
-            regular_p1<ASM, K, NT, NS, 3, SYM><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else if (phase_class == 2)
-            regular_p1<ASM, K, NT, NS, 2, SYM><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else if (phase_class == 1)
-            regular_p1<ASM, K, NT, NS, 1, SYM><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else
-            regular_p1<ASM, K, NT, NS, 0, SYM><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-    }
-}
-
-template <int ASM, int K, int NT, int NS>
-static void launch_p1_shapes(const RegParams &prm, const QuadRule &rule, int phase_class, bool sym, dim3 grid,
-                             cudaStream_t st) {
-    // single layer and hypersingular: symmetric; double / adjoint double layer: each pair
-    // also gives the transposed pair's block from the other normal (p1.cuh)
-    constexpr bool SYMMETRIC_OP = NT == NS;
-    if constexpr (SYMMETRIC_OP) {
-        if (sym) {
-            launch_p1_phase<ASM, K, NT, NS, true>(prm, rule, phase_class, grid, st);
-            return;
-        }
-    }
-    launch_p1_phase<ASM, K, NT, NS, false>(prm, rule, phase_class, grid, st);
-}
-
-// Scalar and hypersingular operators on P1 / DP1 / P0 spaces with the 6-point
-// rule (p1.cuh).
-template <int ASM, int K>
-static cudaError_t launch_p1(const RegParams &prm, const QuadRule &rule, int phase_class, bool sym, cudaStream_t st) {
-    dim3 grid((unsigned)((prm.ntrial + DP0_THREADS - 1) / DP0_THREADS),
-              (unsigned)((prm.ntest + P1_TCHUNK - 1) / P1_TCHUNK));
-    const int nt = prm.tnshape, ns = prm.snshape;
-    if (nt == 3 && ns == 3)
-        launch_p1_shapes<ASM, K, 3, 3>(prm, rule, phase_class, sym, grid, st);
-    else if (nt == 3)
-        launch_p1_shapes<ASM, K, 3, 1>(prm, rule, phase_class, false, grid, st);
-    else if (ns == 3)
-        launch_p1_shapes<ASM, K, 1, 3>(prm, rule, phase_class, false, grid, st);
-    else
-        launch_p1_shapes<ASM, K, 1, 1>(prm, rule, phase_class, sym, grid, st);
-    return cudaGetLastError();
-}
-
 // A <- A + A^T for an n x n matrix with row stride ld, in 32 x 32 tiles: the
 // block of tile pair (bi, bj), bi <= bj, reads both tiles and writes both sums.
 __device__ __forceinline__ double add_pair(double a, double b) { return a + b; }
@@ -489,97 +264,6 @@ static cudaError_t launch_add_transpose(void *a, int64_t n, int64_t ld, bool is_
         add_transpose<double2><<<grid, block, 0, st>>>(reinterpret_cast<double2 *>(a), n, ld);
     else
         add_transpose<double><<<grid, block, 0, st>>>(reinterpret_cast<double *>(a), n, ld);
-    return cudaGetLastError();
-}
-
-// Mixed-precision single layer, double layers and hypersingular on P1 spaces (p1_mixed.cuh): Helmholtz
-// (phase classes, real or complex k), Laplace and modified Helmholtz (no phase classes).
-template <int ASM, int K, bool SYM, bool CK>
-static void p1_mixed_phase(const RegParams &prm, const QuadRule &rule, int phase_class, dim3 grid, cudaStream_t st) {
-    if constexpr (K != BEMPPCUDA_HELMHOLTZ_SLP && K != BEMPPCUDA_HELMHOLTZ_DLP && K != BEMPPCUDA_HELMHOLTZ_ADLP) {
-        regular_p1_mixed<ASM, K, 0, SYM, false><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-    } else {
-        if (phase_class == 2)
-            regular_p1_mixed<ASM, K, 2, SYM, CK><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else if (phase_class == 1)
-            regular_p1_mixed<ASM, K, 1, SYM, CK><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else
-            regular_p1_mixed<ASM, K, 0, SYM, CK><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-    }
-}
-
-// A P0 space beside a P1 one (scalar operators): per-pair sweep, the general phase class.
-template <int K, int NT, int NS>
-static void p1_mixed_pair(const RegParams &prm, const QuadRule &rule, dim3 grid, cudaStream_t st) {
-    constexpr bool helm = K == BEMPPCUDA_HELMHOLTZ_SLP || K == BEMPPCUDA_HELMHOLTZ_DLP || K == BEMPPCUDA_HELMHOLTZ_ADLP;
-    if constexpr (helm) {
-        if (prm.p[1] != 0.0) {
-            regular_p1_mixed<BEMPPCUDA_ASM_SCALAR, K, 0, false, true, NT, NS><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-            return;
-        }
-    }
-    regular_p1_mixed<BEMPPCUDA_ASM_SCALAR, K, 0, false, false, NT, NS><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-}
-
-template <int ASM, int K>
-static cudaError_t launch_p1_mixed(const RegParams &prm, const QuadRule &rule, int phase_class, bool sym,
-                                   cudaStream_t st) {
-    constexpr bool rwg = ASM == BEMPPCUDA_ASM_EFIE || ASM == BEMPPCUDA_ASM_MFIE;
-    dim3 grid((unsigned)((prm.ntrial + DP0_THREADS - 1) / DP0_THREADS),
-              rwg ? lin_row_blocks(prm.ntrial, prm.ntest, sym)
-                  : (unsigned)((prm.ntest + P1_TCHUNK - 1) / P1_TCHUNK));
-    if constexpr (ASM == BEMPPCUDA_ASM_SCALAR) {
-        if (prm.tnshape == 3 && prm.snshape == 1) {
-            p1_mixed_pair<K, 3, 1>(prm, rule, grid, st);
-            return cudaGetLastError();
-        }
-        if (prm.tnshape == 1 && prm.snshape == 3) {
-            p1_mixed_pair<K, 1, 3>(prm, rule, grid, st);
-            return cudaGetLastError();
-        }
-    }
-    constexpr bool helm = K == BEMPPCUDA_HELMHOLTZ_SLP || K == BEMPPCUDA_HELMHOLTZ_DLP ||
-                          K == BEMPPCUDA_HELMHOLTZ_ADLP;
-    const bool ck = helm && prm.p[1] != 0.0;
-    if (ck) {
-        if constexpr (helm) {
-            if (sym)
-                p1_mixed_phase<ASM, K, true, true>(prm, rule, phase_class, grid, st);
-            else
-                p1_mixed_phase<ASM, K, false, true>(prm, rule, phase_class, grid, st);
-        }
-    } else if (sym) {
-        p1_mixed_phase<ASM, K, true, false>(prm, rule, phase_class, grid, st);
-    } else {
-        p1_mixed_phase<ASM, K, false, false>(prm, rule, phase_class, grid, st);
-    }
-    return cudaGetLastError();
-}
-
-// Maxwell electric / magnetic field on RWG / SNC spaces, 6-point rule, real
-// nonzero wavenumber (rwg.cuh).
-template <int ASM>
-static cudaError_t launch_rwg(const RegParams &prm, const QuadRule &rule, int phase_class, bool sym, cudaStream_t st) {
-    dim3 grid((unsigned)((prm.ntrial + DP0_THREADS - 1) / DP0_THREADS), lin_row_blocks(prm.ntrial, prm.ntest, sym));
-    if (sym) {
-        if (phase_class == 3)  // complex wavenumber
-            regular_rwg<ASM, 3, true><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else if (phase_class == 2)
-            regular_rwg<ASM, 2, true><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else if (phase_class == 1)
-            regular_rwg<ASM, 1, true><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else
-            regular_rwg<ASM, 0, true><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-    } else {
-        if (phase_class == 3)
-            regular_rwg<ASM, 3, false><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else if (phase_class == 2)
-            regular_rwg<ASM, 2, false><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else if (phase_class == 1)
-            regular_rwg<ASM, 1, false><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-        else
-            regular_rwg<ASM, 0, false><<<grid, DP0_THREADS, 0, st>>>(prm, rule);
-    }
     return cudaGetLastError();
 }
 
@@ -680,6 +364,15 @@ int bc_regular_launch(const bemppcuda_regular_args *a, cudaStream_t st) {
     // 1/2 lets the sine / cosine skip the range reduction (classes 1, 2)
     const double theta = fabs(a->params[0]) * a->phase_radius;
     const int phase_class = a->phase_radius > 0.0 ? (theta <= 0.5 ? 2 : (theta <= 1.0 ? 1 : 0)) : 0;
+    // the orbit form of the P1 and RWG sweeps takes the two-orbit rule (any other 6-point rule goes to the points form
+    // where the operator has one, else to regular_generic in FP64); the offset class bounds |k| |r - r_c|, of a
+    // complex wavenumber by the larger of its parts
+    OrbitRule orbit = {};
+    const bool orbits = orbit_rule(rule, orbit);
+    const OrbitConsts oc = orbits ? orbit_consts(orbit) : OrbitConsts{};
+    const double im_k = a->kernel >= BEMPPCUDA_MODHELM_SLP && a->kernel <= BEMPPCUDA_MODHELM_ADLP ? 0.0 : fabs(a->params[1]);
+    const int cls = a->kernel <= BEMPPCUDA_LAPLACE_ADLP
+                        ? 0 : offset_class64(fmax(fabs(a->params[0]), im_k) * a->phase_radius * (orbits ? orbit.rho : 1.0));
     // one DP0 space on both sides of one grid: each element pair gives A_ij and A_ji
     const bool sym = dp0 && !a->no_symmetry && a->grids_identical && a->test.support == a->trial.support &&
                      a->test.nsupport == a->trial.nsupport && a->test_grid.geom == a->trial_grid.geom &&
@@ -720,21 +413,15 @@ int bc_regular_launch(const bemppcuda_regular_args *a, cudaStream_t st) {
         prm.col0 = a->col_begin;
     }
     if (dp0) {
-        switch (a->kernel) {
-        case BEMPPCUDA_LAPLACE_SLP: err = launch_dp0<BEMPPCUDA_LAPLACE_SLP>(prm, rule, mixed, phase_class, sym, row0, row1, st); break;
-        case BEMPPCUDA_LAPLACE_DLP: err = launch_dp0<BEMPPCUDA_LAPLACE_DLP>(prm, rule, mixed, phase_class, sym, row0, row1, st); break;
-        case BEMPPCUDA_LAPLACE_ADLP: err = launch_dp0<BEMPPCUDA_LAPLACE_ADLP>(prm, rule, mixed, phase_class, sym, row0, row1, st); break;
-        case BEMPPCUDA_HELMHOLTZ_SLP: err = launch_dp0<BEMPPCUDA_HELMHOLTZ_SLP>(prm, rule, mixed, phase_class, sym, row0, row1, st); break;
-        case BEMPPCUDA_HELMHOLTZ_DLP: err = launch_dp0<BEMPPCUDA_HELMHOLTZ_DLP>(prm, rule, mixed, phase_class, sym, row0, row1, st); break;
-        case BEMPPCUDA_HELMHOLTZ_ADLP: err = launch_dp0<BEMPPCUDA_HELMHOLTZ_ADLP>(prm, rule, mixed, phase_class, sym, row0, row1, st); break;
-        case BEMPPCUDA_MODHELM_SLP: err = launch_dp0<BEMPPCUDA_MODHELM_SLP>(prm, rule, mixed, phase_class, sym, row0, row1, st); break;
-        case BEMPPCUDA_MODHELM_DLP: err = launch_dp0<BEMPPCUDA_MODHELM_DLP>(prm, rule, mixed, phase_class, sym, row0, row1, st); break;
-        case BEMPPCUDA_MODHELM_ADLP: err = launch_dp0<BEMPPCUDA_MODHELM_ADLP>(prm, rule, mixed, phase_class, sym, row0, row1, st); break;
-        case BEMPPCUDA_HELMHOLTZ_COMBINED: err = launch_dp0<BEMPPCUDA_HELMHOLTZ_COMBINED>(prm, rule, mixed, phase_class, sym, row0, row1, st); break;
-        default: bc_set_error("kernel %d not valid for boundary assembly", a->kernel); return BEMPPCUDA_ERR_INVALID;
+        if (a->kernel > BEMPPCUDA_MODHELM_ADLP && a->kernel != BEMPPCUDA_HELMHOLTZ_COMBINED) {
+            bc_set_error("kernel %d not valid for boundary assembly", a->kernel);
+            return BEMPPCUDA_ERR_INVALID;
         }
+        err = launch_dp0_kernel(a->kernel, prm, rule, oc, sym_form(a->kernel, prm.p, a->phase_radius, orbits, orbit), mixed,
+                                phase_class, sym, row0, row1, st);
     } else if ((a->assembly == BEMPPCUDA_ASM_EFIE || a->assembly == BEMPPCUDA_ASM_MFIE) && a->nq == NQ6 &&
-               !a->overwrite && a->kernel == BEMPPCUDA_HELMHOLTZ_SLP && (a->params[0] != 0.0 || a->params[1] != 0.0) &&
+               (orbits || (!mixed && a->params[1] == 0.0)) && !a->overwrite &&
+               a->kernel == BEMPPCUDA_HELMHOLTZ_SLP && (a->params[0] != 0.0 || a->params[1] != 0.0) &&
                a->test.shapeset == BEMPPCUDA_SHAPE_RWG && a->trial.shapeset == BEMPPCUDA_SHAPE_RWG &&
                a->test.nshape == 3 && a->trial.nshape == 3) {
         // RWG and SNC share their dof maps; the caller passes the same arrays for both
@@ -742,21 +429,17 @@ int bc_regular_launch(const bemppcuda_regular_args *a, cudaStream_t st) {
                           a->test.l2g == a->trial.l2g && a->test.mult == a->trial.mult &&
                           a->test.nsupport == a->trial.nsupport && a->test_grid.geom == a->trial_grid.geom &&
                           prm.ntest == prm.ntrial;
-        // a complex wavenumber takes phase class 3 (exp(-Im k r) per point pair)
-        const int rwg_phase = a->params[1] != 0.0 ? 3 : phase_class;
-        if (mixed && rwg_mixed && a->assembly == BEMPPCUDA_ASM_EFIE)
-            err = launch_p1_mixed<BEMPPCUDA_ASM_EFIE, BEMPPCUDA_HELMHOLTZ_SLP>(prm, rule, phase_class, rsym, st);
-        else if (mixed && rwg_mixed)
-            err = launch_p1_mixed<BEMPPCUDA_ASM_MFIE, BEMPPCUDA_HELMHOLTZ_SLP>(prm, rule, phase_class, rsym, st);
-        else if (a->assembly == BEMPPCUDA_ASM_EFIE)
-            err = launch_rwg<BEMPPCUDA_ASM_EFIE>(prm, rule, rwg_phase, rsym, st);
+        if (mixed && rwg_mixed)
+            err = launch_p1_mixed_kernel(a->assembly, a->kernel, prm, rule, phase_class, rsym, st);
         else
-            err = launch_rwg<BEMPPCUDA_ASM_MFIE>(prm, rule, rwg_phase, rsym, st);
+            err = launch_rwg_kernel(a->assembly, prm, rule, oc, cls, rsym, st);
     } else if (const bool psym = !a->no_symmetry && a->grids_identical && a->test.support == a->trial.support &&
                                  a->test.l2g == a->trial.l2g && a->test.mult == a->trial.mult &&
                                  a->test.nsupport == a->trial.nsupport && a->test_grid.geom == a->trial_grid.geom &&
                                  a->test.normal_mult == a->trial.normal_mult && prm.ntest == prm.ntrial;
-               a->nq == NQ6 && !a->overwrite && a->test.shapeset != BEMPPCUDA_SHAPE_RWG &&
+               a->nq == NQ6 && (orbits || (!mixed && p1_points_form(a->assembly, a->kernel, a->params))) &&
+               !a->overwrite &&
+               a->test.shapeset != BEMPPCUDA_SHAPE_RWG &&
                a->trial.shapeset != BEMPPCUDA_SHAPE_RWG &&
                ((a->assembly == BEMPPCUDA_ASM_SCALAR && a->kernel <= BEMPPCUDA_MODHELM_ADLP) ||
                 a->assembly == BEMPPCUDA_ASM_LAPLACE_HYP || a->assembly == BEMPPCUDA_ASM_HELM_HYP ||
@@ -768,52 +451,10 @@ int bc_regular_launch(const bemppcuda_regular_args *a, cudaStream_t st) {
                            (a->assembly != BEMPPCUDA_ASM_SCALAR || a->kernel == BEMPPCUDA_LAPLACE_SLP ||
                             a->kernel == BEMPPCUDA_HELMHOLTZ_SLP || a->kernel == BEMPPCUDA_MODHELM_SLP);
         prm.defer_transpose = defer ? 1 : 0;
-        // a complex wavenumber takes phase class 3 (no centroid factoring, exp(-Im k r) per point)
-        const int p1_phase = a->params[1] != 0.0 ? 3 : phase_class;
-        if (mixed && p1_mixed) {
-            if (a->assembly == BEMPPCUDA_ASM_HELM_HYP)
-                err = launch_p1_mixed<BEMPPCUDA_ASM_HELM_HYP, BEMPPCUDA_HELMHOLTZ_SLP>(prm, rule, phase_class, psym, st);
-            else if (a->assembly == BEMPPCUDA_ASM_LAPLACE_HYP)
-                err = launch_p1_mixed<BEMPPCUDA_ASM_LAPLACE_HYP, BEMPPCUDA_LAPLACE_SLP>(prm, rule, 0, psym, st);
-            else if (a->assembly == BEMPPCUDA_ASM_MODHELM_HYP)
-                err = launch_p1_mixed<BEMPPCUDA_ASM_MODHELM_HYP, BEMPPCUDA_MODHELM_SLP>(prm, rule, 0, psym, st);
-            else if (a->kernel == BEMPPCUDA_LAPLACE_SLP)
-                err = launch_p1_mixed<BEMPPCUDA_ASM_SCALAR, BEMPPCUDA_LAPLACE_SLP>(prm, rule, 0, psym, st);
-            else if (a->kernel == BEMPPCUDA_LAPLACE_DLP)
-                err = launch_p1_mixed<BEMPPCUDA_ASM_SCALAR, BEMPPCUDA_LAPLACE_DLP>(prm, rule, 0, psym, st);
-            else if (a->kernel == BEMPPCUDA_LAPLACE_ADLP)
-                err = launch_p1_mixed<BEMPPCUDA_ASM_SCALAR, BEMPPCUDA_LAPLACE_ADLP>(prm, rule, 0, psym, st);
-            else if (a->kernel == BEMPPCUDA_MODHELM_SLP)
-                err = launch_p1_mixed<BEMPPCUDA_ASM_SCALAR, BEMPPCUDA_MODHELM_SLP>(prm, rule, 0, psym, st);
-            else if (a->kernel == BEMPPCUDA_MODHELM_DLP)
-                err = launch_p1_mixed<BEMPPCUDA_ASM_SCALAR, BEMPPCUDA_MODHELM_DLP>(prm, rule, 0, psym, st);
-            else if (a->kernel == BEMPPCUDA_MODHELM_ADLP)
-                err = launch_p1_mixed<BEMPPCUDA_ASM_SCALAR, BEMPPCUDA_MODHELM_ADLP>(prm, rule, 0, psym, st);
-            else if (a->kernel == BEMPPCUDA_HELMHOLTZ_DLP)
-                err = launch_p1_mixed<BEMPPCUDA_ASM_SCALAR, BEMPPCUDA_HELMHOLTZ_DLP>(prm, rule, phase_class, psym, st);
-            else if (a->kernel == BEMPPCUDA_HELMHOLTZ_ADLP)
-                err = launch_p1_mixed<BEMPPCUDA_ASM_SCALAR, BEMPPCUDA_HELMHOLTZ_ADLP>(prm, rule, phase_class, psym, st);
-            else
-                err = launch_p1_mixed<BEMPPCUDA_ASM_SCALAR, BEMPPCUDA_HELMHOLTZ_SLP>(prm, rule, phase_class, psym, st);
-        } else if (a->assembly == BEMPPCUDA_ASM_LAPLACE_HYP) {
-            err = launch_p1<BEMPPCUDA_ASM_LAPLACE_HYP, BEMPPCUDA_LAPLACE_SLP>(prm, rule, p1_phase, psym, st);
-        } else if (a->assembly == BEMPPCUDA_ASM_HELM_HYP) {
-            err = launch_p1<BEMPPCUDA_ASM_HELM_HYP, BEMPPCUDA_HELMHOLTZ_SLP>(prm, rule, p1_phase, psym, st);
-        } else if (a->assembly == BEMPPCUDA_ASM_MODHELM_HYP) {
-            err = launch_p1<BEMPPCUDA_ASM_MODHELM_HYP, BEMPPCUDA_MODHELM_SLP>(prm, rule, p1_phase, psym, st);
-        } else {
-            switch (a->kernel) {
-            case BEMPPCUDA_LAPLACE_SLP: err = launch_p1<0, BEMPPCUDA_LAPLACE_SLP>(prm, rule, p1_phase, psym, st); break;
-            case BEMPPCUDA_LAPLACE_DLP: err = launch_p1<0, BEMPPCUDA_LAPLACE_DLP>(prm, rule, p1_phase, psym, st); break;
-            case BEMPPCUDA_LAPLACE_ADLP: err = launch_p1<0, BEMPPCUDA_LAPLACE_ADLP>(prm, rule, p1_phase, psym, st); break;
-            case BEMPPCUDA_HELMHOLTZ_SLP: err = launch_p1<0, BEMPPCUDA_HELMHOLTZ_SLP>(prm, rule, p1_phase, psym, st); break;
-            case BEMPPCUDA_HELMHOLTZ_DLP: err = launch_p1<0, BEMPPCUDA_HELMHOLTZ_DLP>(prm, rule, p1_phase, psym, st); break;
-            case BEMPPCUDA_HELMHOLTZ_ADLP: err = launch_p1<0, BEMPPCUDA_HELMHOLTZ_ADLP>(prm, rule, p1_phase, psym, st); break;
-            case BEMPPCUDA_MODHELM_SLP: err = launch_p1<0, BEMPPCUDA_MODHELM_SLP>(prm, rule, p1_phase, psym, st); break;
-            case BEMPPCUDA_MODHELM_DLP: err = launch_p1<0, BEMPPCUDA_MODHELM_DLP>(prm, rule, p1_phase, psym, st); break;
-            default: err = launch_p1<0, BEMPPCUDA_MODHELM_ADLP>(prm, rule, p1_phase, psym, st); break;
-            }
-        }
+        if (mixed && p1_mixed)
+            err = launch_p1_mixed_kernel(a->assembly, a->kernel, prm, rule, phase_class, psym, st);
+        else
+            err = launch_p1_kernel(a->assembly, a->kernel, prm, rule, oc, cls, psym, st);
         if (defer && err == cudaSuccess) err = launch_add_transpose(prm.result, a->test.ndofs, prm.ld, prm.is_complex, st);
     } else {
         switch (a->assembly) {

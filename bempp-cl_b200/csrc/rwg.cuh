@@ -26,10 +26,9 @@
 //          B(p) = sum_q H (w_s(q) x d),  C(p) = sum_q H d,
 //          MFIE_ij = PB - c_sj . PC - c_ti . QB + c_ti . (c_sj x QC),
 //        PB = sum_p w_t(p) . B(p), PC = sum_p C(p) x w_t(p), QB = sum_p B(p), QC = sum_p C(p).
-// exp(ikr) is factored about the centroid distance as in the DP0 / P1 kernels
-// (phase classes 1, 2).  Class 3 is a complex wavenumber k = kr + i ki:
-// exp(ikr) = exp(i kr r) exp(-ki r) per point pair, (ikr - 1) = -(1 + ki r) + i kr r,
-// and -ik, -4 / (ik) = 4i conj(k) / |k|^2 as complex factors per element pair.
+// In the orbit form the moments are orbit_moments (orbit_pair.cuh) of the linear shape functions, whose sums give
+// those of {1, xi, eta}.  A complex wavenumber k = kr + i ki: -ik, -4 / (ik) = 4i conj(k) / |k|^2 as complex factors
+// per element pair.
 // SYM (test and trial spaces with the same dof maps on one grid, as RWG and
 // SNC are): both operators are symmetric under exchanging the pair's
 // elements (G is symmetric; for MFIE both d and the cross product change
@@ -37,16 +36,16 @@
 #pragma once
 
 #include "dp0.cuh"
+#include "orbit_pair.cuh"
 
 namespace bc {
 
 constexpr int RWG_TCHUNK = 32;
 
 struct TestBlockRWG {
-    double x[RWG_TCHUNK][NQ6][3];
+    OrbitTest o[RWG_TCHUNK];
     double j0[RWG_TCHUNK][3];
     double j1[RWG_TCHUNK][3];
-    double c[RWG_TCHUNK][3];
     double v0[RWG_TCHUNK][3];   // vertex 0 (MFIE moments)
     double fac[RWG_TCHUNK][3];  // edge length times multiplier of each test function
     int64_t row[RWG_TCHUNK][3];
@@ -223,12 +222,26 @@ __device__ __forceinline__ void mfie_block_moments(const double mre[3][3], const
     }
 }
 
-template <int ASM, int PHC, bool SYM>
-__global__ void __launch_bounds__(DP0_THREADS) regular_rwg(RegParams prm, QuadRule rule) {
+struct TestBlockRWGPoints {
+    double x[RWG_TCHUNK][NQ6][3];
+    double j0[RWG_TCHUNK][3];
+    double j1[RWG_TCHUNK][3];
+    double c[RWG_TCHUNK][3];
+    double v0[RWG_TCHUNK][3];   // vertex 0 (MFIE moments)
+    double fac[RWG_TCHUNK][3];  // edge length times multiplier of each test function
+    int64_t row[RWG_TCHUNK][3];
+    int v[RWG_TCHUNK][3];
+};
+
+// Real wavenumber, any 6-point rule: coordinates differenced per point pair, moments of {1, xi, eta} directly.  The
+// orbit sums below take fewer FP64 operations but leave the FP64 pipe emptier (47 against 52 %, 36 scattered atomic
+// adds per pair behind either): 4608 elements, k = 2, electric field 2.05 ms against 1.96 here, magnetic 2.08
+// against 1.98.  CLS: offset class (fastmath.cuh).
+template <int ASM, int CLS, bool SYM>
+__global__ void __launch_bounds__(DP0_THREADS) regular_rwg_points(RegParams prm, QuadRule rule) {
     constexpr bool EFIE = ASM == BEMPPCUDA_ASM_EFIE;
-    constexpr bool PH = PHC == 1 || PHC == 2;
-    constexpr bool CK = PHC == 3;
-    __shared__ TestBlockRWG sb;
+    constexpr bool PH = CLS > 0;
+    __shared__ TestBlockRWGPoints sb;
 
     // test elements per CTA: ceil(ntest / gridDim.y) <= RWG_TCHUNK (the launch picks the row blocks)
     const int rows = (int)((prm.ntest + gridDim.y - 1) / gridDim.y);
@@ -279,7 +292,7 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_rwg(RegParams prm, QuadRu
         scol[j] = prm.sl2g[s * 3 + j];
         sfac[j] = prm.smult[s * 3 + j] * edge_length(prm.sg, prm.sne, s, j);
     }
-    const double kr = prm.p[0], ki = CK ? prm.p[1] : 0.0;
+    const double kr = prm.p[0];
 
     for (int tt = 0; tt < tcount; ++tt) {
         if (SYM && t0 + tt >= si) break;  // rows increase with tt
@@ -310,18 +323,8 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_rwg(RegParams prm, QuadRu
                 const double rinv = rsqrt64(r2);
                 const double r = r2 * rinv;
                 double sn, cs;
-                if (PH && PHC == 2)
-                    sincos_half64(fma(kr, r, -krc), &sn, &cs);
-                else if (PH)
-                    sincos_small64(fma(kr, r, -krc), &sn, &cs);
-                else
-                    sincos_cw64(kr * r, &sn, &cs);
-                if (CK) {
-                    const double am = exp(-ki * r);
-                    sn *= am;
-                    cs *= am;
-                }
-                // EFIE: G 4 pi = (cs + i sn) / r; MFIE: H 4 pi = (cs + i sn)(-(1 + ki r) + i k r) / r^3
+                sincos_off64<CLS>(fma(kr, r, -krc), &sn, &cs);
+                // EFIE: G 4 pi = (cs + i sn) / r; MFIE: H 4 pi = (cs + i sn)(-1 + i k r) / r^3
                 // (the phase exp(ik r_c) and 1 / (4 pi) are applied per pair)
                 double gr, gi;
                 if (EFIE) {
@@ -329,9 +332,8 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_rwg(RegParams prm, QuadRu
                     gi = sn * rinv;
                 } else {
                     const double f = rinv * rinv * rinv, kq = kr * r;
-                    const double a = CK ? fma(ki, r, 1.0) : 1.0;
-                    gr = -fma(kq, sn, a * cs) * f;
-                    gi = fma(kq, cs, -a * sn) * f;
+                    gr = -fma(kq, sn, cs) * f;
+                    gi = fma(kq, cs, -sn) * f;
                 }
                 const double v[3] = {rule.w[q], rule.sw[q][1], rule.sw[q][2]};  // w_q (1, xi_q, eta_q)
 #pragma unroll
@@ -351,7 +353,7 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_rwg(RegParams prm, QuadRu
         }
         double blk_re[3][3], blk_im[3][3];
         if (EFIE) {
-            efie_block<CK>(mre, mim, tj0, tj1, gs.j0, gs.j1, kr, ki, blk_re, blk_im);
+            efie_block<false>(mre, mim, tj0, tj1, gs.j0, gs.j1, kr, 0.0, blk_re, blk_im);
         } else {
             const double tv0[3] = {sb.v0[tt][0], sb.v0[tt][1], sb.v0[tt][2]};
             mfie_block_moments(mre, mim, tv0, tj0, tj1, gs.v0, gs.j0, gs.j1, blk_re, blk_im);
@@ -378,6 +380,128 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_rwg(RegParams prm, QuadRu
                     double *ot = reinterpret_cast<double *>(prm.result) + 2 * (scol[j] * prm.ld + row);
                     atomicAdd(ot, vr * m);
                     atomicAdd(ot + 1, vi * m);
+                }
+            }
+        }
+    }
+}
+
+// Complex wavenumber, two-orbit rule (orbit_pair.cuh): the amplitude exp(-Im k r) split about the centroid distance
+// like the phase (4608 elements, k = 2 + 0.2i: electric field 2.96 -> 2.24 ms, magnetic 3.67 -> 2.37 ms).
+template <int ASM, int CLS, bool SYM>
+__global__ void __launch_bounds__(DP0_THREADS) regular_rwg_orbit(RegParams prm, OrbitConsts oc) {
+    constexpr bool CK = true;
+    constexpr bool EFIE = ASM == BEMPPCUDA_ASM_EFIE;
+    __shared__ TestBlockRWG sb;
+    // the trial element's fields, then vertex 0, the edge lengths times multipliers and the dofs
+    constexpr int V0 = OT_FIELDS, FAC = V0 + 3, COL = FAC + 3, FIELDS = COL + 3;
+    __shared__ double park[FIELDS][DP0_THREADS];
+
+    // test elements per CTA: ceil(ntest / gridDim.y) <= RWG_TCHUNK (the launch picks the row blocks)
+    const int rows = (int)((prm.ntest + gridDim.y - 1) / gridDim.y);
+    const int64_t t0 = (int64_t)blockIdx.y * rows;
+    if (SYM && t0 >= ((int64_t)blockIdx.x + 1) * DP0_THREADS) return;  // below the diagonal
+    const int tcount = (int)min((int64_t)rows, prm.ntest - t0);
+    for (int idx = threadIdx.x; idx < tcount; idx += blockDim.x) {
+        const int64_t t = prm.tsup[t0 + idx];
+        Geom g;
+        load_geom(prm.tg, prm.tne, t, 1.0, g);
+        stage_orbit(prm.tg, prm.tne, t, g, oc, sb.o[idx]);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            sb.j0[idx][d] = g.j0[d];
+            sb.j1[idx][d] = g.j1[d];
+            sb.v0[idx][d] = g.v0[d];
+            sb.v[idx][d] = __ldg(prm.tel + 3 * t + d);
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            sb.fac[idx][i] = prm.tmult[t * 3 + i] * edge_length(prm.tg, prm.tne, t, i);
+            sb.row[idx][i] = prm.tl2g[t * 3 + i];
+        }
+    }
+    __syncthreads();
+
+    const int64_t si = (int64_t)blockIdx.x * DP0_THREADS + threadIdx.x;
+    if (si >= prm.ntrial) return;
+    const int64_t s = prm.ssup[si];
+    Geom gs;
+    load_geom(prm.sg, prm.sne, s, 1.0, gs);
+    const int sv0 = __ldg(prm.sel + 3 * s), sv1 = __ldg(prm.sel + 3 * s + 1), sv2 = __ldg(prm.sel + 3 * s + 2);
+    const OrbitTrial<DP0_THREADS> tr = park_orbit_trial<DP0_THREADS>(prm.sg, prm.sne, s, gs, &park[0][0]);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        park[V0 + j][threadIdx.x] = gs.v0[j];
+        park[FAC + j][threadIdx.x] = prm.smult[s * 3 + j] * edge_length(prm.sg, prm.sne, s, j);
+        park[COL + j][threadIdx.x] = __longlong_as_double((int64_t)prm.sl2g[s * 3 + j]);
+    }
+    const double kr = prm.p[0], ki = prm.p[1];
+
+#pragma unroll 1
+    for (int tt = 0; tt < tcount; ++tt) {
+        if (SYM && t0 + tt >= si) break;  // rows increase with tt
+        if (prm.grids_identical && shares_vertex(sb.v[tt], sv0, sv1, sv2)) continue;
+        OrbitPair pair;
+        orbit_pair<FAM_HELM, CK, CLS>(sb.o[tt], tr, oc, kr, ki, pair);
+        // moments of K = G (EFIE) or H = G (ikr - 1) / r^2 (MFIE), both times 4 pi and without the pair's
+        // phase factor: of the linear shape functions, then of {1, xi, eta} (1 = their sum, xi and eta the
+        // second and third)
+        double lre[3][3], lim[3][3], mre[3][3], mim[3][3];
+        orbit_moments<!EFIE, FAM_HELM, CK, CLS, 3, 3>(sb.o[tt], tr, pair, oc, kr, ki, lre, lim);
+#pragma unroll
+        for (int a = 1; a < 3; ++a) {
+#pragma unroll
+            for (int b = 1; b < 3; ++b) {
+                mre[a][b] = lre[a][b];
+                mim[a][b] = lim[a][b];
+            }
+            mre[a][0] = lre[a][0] + lre[a][1] + lre[a][2];
+            mim[a][0] = lim[a][0] + lim[a][1] + lim[a][2];
+            mre[0][a] = lre[0][a] + lre[1][a] + lre[2][a];
+            mim[0][a] = lim[0][a] + lim[1][a] + lim[2][a];
+        }
+        mre[0][0] = lre[0][0] + lre[0][1] + lre[0][2] + mre[1][0] + mre[2][0];
+        mim[0][0] = lim[0][0] + lim[0][1] + lim[0][2] + mim[1][0] + mim[2][0];
+        const double tj0[3] = {sb.j0[tt][0], sb.j0[tt][1], sb.j0[tt][2]};
+        const double tj1[3] = {sb.j1[tt][0], sb.j1[tt][1], sb.j1[tt][2]};
+        // Jacobian columns f_1 - f_0, f_2 - f_0 = -2 f_0 - f_1
+        double f0[3], f1[3], sj0[3], sj1[3];
+        tr.f(f0, f1);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            sj0[d] = f1[d] - f0[d];
+            sj1[d] = -fma(2.0, f0[d], f1[d]);
+        }
+        double blk_re[3][3], blk_im[3][3];
+        if (EFIE) {
+            efie_block<CK>(mre, mim, tj0, tj1, sj0, sj1, kr, ki, blk_re, blk_im);
+        } else {
+            const double tv0[3] = {sb.v0[tt][0], sb.v0[tt][1], sb.v0[tt][2]};
+            const double sv[3] = {tr.ld(V0), tr.ld(V0 + 1), tr.ld(V0 + 2)};
+            mfie_block_moments(mre, mim, tv0, tj0, tj1, sv, sj0, sj1, blk_re, blk_im);
+        }
+        double ph_c, ph_s;
+        orbit_phase<FAM_HELM, CK, CLS>(pair, ph_c, ph_s);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const double ft = sb.fac[tt][i] * BC_INV_4PI;
+            if (ft == 0.0) continue;
+            const int64_t row = sb.row[tt][i];
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const double m = ft * tr.ld(FAC + j);
+                if (m == 0.0) continue;
+                const double cm = ph_c * m, sm = ph_s * m;
+                const double vr = fma(blk_re[i][j], cm, -blk_im[i][j] * sm);
+                const double vi = fma(blk_re[i][j], sm, blk_im[i][j] * cm);
+                const int64_t col = tr.li(COL + j);
+                double *o = reinterpret_cast<double *>(prm.result) + 2 * (row * prm.ld + col);
+                atomicAdd(o, vr);
+                atomicAdd(o + 1, vi);
+                if (SYM) {
+                    double *ot = reinterpret_cast<double *>(prm.result) + 2 * (col * prm.ld + row);
+                    atomicAdd(ot, vr);
+                    atomicAdd(ot + 1, vi);
                 }
             }
         }
