@@ -82,9 +82,9 @@ __device__ __forceinline__ void run_tile_sym(const BatchDev &P, const QuadRule &
                                              int orbits, int64_t tx, int64_t ty, TileShared &sh) {
     const int64_t t0 = ty * P.rows;
     const int rows = P.rows;
-    if (P.precision == BEMPPCUDA_FP64) {
-        // a launch whose rule is not the two-orbit one (the problems were prepared with one that is) takes the
-        // unfactored points form
+    // (the mixed sweep is written for the two-orbit rule: any other rule runs in FP64)
+    if (P.precision == BEMPPCUDA_FP64 || !orbits) {
+        // a launch whose rule is not the one that the problems were prepared with takes the unfactored points form
         switch (orbits == P.orbits ? P.form : P.ck ? SYM_POINTS_CK : SYM_POINTS) {
 #define BC_BATCH_FORM(F)                                                                                    \
     case F:                                                                                                 \

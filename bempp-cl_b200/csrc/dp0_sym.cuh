@@ -404,14 +404,13 @@ __device__ __forceinline__ void regular_dp0_fp64_sym_tile(const RegParams &prm, 
 
 namespace bc {
 
-// Test block of the packed symmetric sweep: per test point the scaled offset
-// o = kappa (x_p - c_t) as -2 o, each component stored twice so that it is an
-// f32x2 operand straight from shared memory, and |o|^2.
+// Test block of the packed symmetric sweep, lengths in units of 1/kappa: vertex offsets e_i = kappa (v_i - c_t),
+// -g_o^2 |e_i|^2 / 2 per orbit, centroid, normal.
 struct TestBlock32q {
-    float4 mxy[DP0_TCHUNK][NQ6];  // (-2 o_x, -2 o_x, -2 o_y, -2 o_y)
-    float4 mzw[DP0_TCHUNK][NQ6];  // (-2 o_z, -2 o_z, |o|^2, |o|^2)
-    double c[DP0_TCHUNK][3];      // centroid
-    float4 n[DP0_TCHUNK];         // unit normal (fourth entry unused)
+    float e[DP0_TCHUNK][3][3];
+    float hge[DP0_TCHUNK][2][3];
+    double c[DP0_TCHUNK][3];
+    float4 n[DP0_TCHUNK];  // unit normal (fourth entry unused)
     double ie[DP0_TCHUNK];
     int v[DP0_TCHUNK][3];
 };
@@ -446,19 +445,25 @@ __device__ __forceinline__ void sincos2_sym(float2 x, float2 *s, float2 *c) {
     }
 }
 
-// Packed mixed precision in wavenumber-scaled units (as regular_dp0_mixed2_tile).
-// Per point pair, with g = w (d'.n) / r'^2 and the shared factors
-// h1 = cos / r' + sin, h2 = cos - sin / r', the double-layer part of an entry
-// is -g h1 + i g h2 (times kappa^2); the two entries differ only in (d'.n).
+// Packed mixed precision in wavenumber-scaled units with the two-orbit rule (orbit.cuh).  The trial points of
+// one vertex, one of each orbit, travel together in f32x2 operations, so an orbit's weight is applied to its
+// half of the sums at the end of the pair, and the offset products need one dot product per pair of vertices:
+//   s = r'^2 - r_c'^2 = A_q + B_p - 2 g_p g_q e_i . f_j,
+//   A_q = g_q^2 |f_j|^2 + 2 g_q D . f_j,  B_p = g_p^2 |e_i|^2 - 2 g_p D . e_i.
+// 1/r' by rsqrt.approx.  The phase offset theta = r' - r_c' would lose its accuracy in the subtraction (r' is
+// good to 1e-7 r', up to 2e-6 at r' = 20); one Newton step on theta^2 + 2 r_c' theta = s from it,
+//   theta = t + (s - t (t + 2 r_c')) / (2 r'),  t = r'^2 (1 / r') - r_c',
+// restores it to rounding of theta itself, in four packed operations in place of the reciprocal
+// 1 / (r' + r_c') of the special-function unit, which with the square root and the cosine bounded the sweep
+// beside the FMA pipe.  (The code carries -theta and -s / 2: f32x2 operations have no negation.)
+// Per point pair, with g = w (d'.n) / r'^2 and the shared factors h1 = cos / r' + sin, h2 = cos - sin / r', the
+// double-layer part of an entry is -g h1 + i g h2 (times kappa^2); the two entries differ only in (d'.n).
 //
-// Per element pair: the centroid offset D and |D|^2 in FP64 (r_c' for the
-// phase), FP32 copies for the point-pair terms; elements whose centroids are
-// farther apart than prm.near_r cannot share a vertex, so the vertex test
-// runs only for near pairs; the pair phase exp(i r_c') by phase_reduced32.
-// The six test points form two orbits of equal weight (w_a for points 0-2,
-// w_b for 3-5, the order-4 rule): the FP32 sums of the first orbit are scaled
-// by w_a / w_b when the second begins, and everything is converted to FP64
-// once, times w_b.
+// Per element pair: the centroid offset D and |D|^2 in FP64 (r_c' for the phase), FP32 copies for the
+// point-pair terms; elements whose centroids are farther apart than prm.near_r cannot share a vertex, so the
+// vertex test runs only for near pairs; the pair phase exp(i r_c') by phase_reduced32.  The FP32 sums of the
+// first test orbit are scaled by w_a / w_b when the second begins, and everything is converted to FP64 once,
+// times w_b.
 // CK: a complex wavenumber k = kr + i ki in units of 1/kr: the amplitude e^{-beta r'} (beta = ki / kr)
 // split like the phase, e^{-beta theta} per point pair by __expf and e^{-beta r_c'} per element pair by
 // exp_neg_reduced; the double-layer factor (i k r - 1) = -(1 + beta r') + i r' turns 1 / r' into
@@ -468,32 +473,30 @@ __device__ __forceinline__ void regular_dp0_mixed_sym_tile(const RegParams &prm,
                                                          int64_t tile_x, int64_t t0, int rows, TestBlock32q &sb) {
     using ST = SymTraits<K>;
     static_assert(!CK || ST::helm, "complex wavenumber: the Helmholtz kernels");
-    constexpr int NP = NQ6 / 2;
     // units of 1/kappa: Re k (Helmholtz), omega (modified Helmholtz), 1 (Laplace); callers guarantee kappa > 0
     const double kap = ST::helm || ST::modhelm ? prm.p[0] : 1.0;
     const double betd = CK ? prm.p[1] / prm.p[0] : 0.0;
     const float2 bet2 = b2((float)betd);
+    // the orbits' offset factors: the first point of an orbit belongs to vertex 2
+    const double g0d = 1.0 - 3.0 * rule.x[0], g1d = 1.0 - 3.0 * rule.x[NQ6 / 2];
+    const float go[2] = {(float)g0d, (float)g1d};
+    const float2 g2 = f2(go[0], go[1]);
     const int tcount = (int)min((int64_t)rows, prm.ntest - t0);
     for (int idx = threadIdx.x; idx < tcount; idx += blockDim.x) {
         const int64_t t = prm.tsup[t0 + idx];
         Geom g;
         load_geom(prm.tg, prm.tne, t, prm.tnm ? (double)prm.tnm[t] : 1.0, g);
-        double c[3];
+        double e[3][3];
+        orbit_offsets(g, e);
 #pragma unroll
-        for (int d = 0; d < 3; ++d) c[d] = __ldg(prm.tg + (22 + d) * prm.tne + t);
-        for (int p = 0; p < NQ6; ++p) {
-            double x[3];
-            to_global(g, rule.x[p], rule.y[p], x);
-            const float o0 = (float)(kap * (x[0] - c[0])), o1 = (float)(kap * (x[1] - c[1])),
-                        o2 = (float)(kap * (x[2] - c[2]));
-            const float m2 = fmaf(o2, o2, fmaf(o1, o1, o0 * o0));
-            sb.mxy[idx][p] = make_float4(-2.f * o0, -2.f * o0, -2.f * o1, -2.f * o1);
-            sb.mzw[idx][p] = make_float4(-2.f * o2, -2.f * o2, m2, m2);
-        }
+        for (int i = 0; i < 3; ++i) {
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            sb.c[idx][d] = c[d];
-            sb.v[idx][d] = __ldg(prm.tel + 3 * t + d);
+            for (int d = 0; d < 3; ++d) sb.e[idx][i][d] = (float)(kap * e[i][d]);
+            const double m = kap * kap * odot(e[i], e[i]);
+            sb.hge[idx][0][i] = (float)(-0.5 * g0d * g0d * m);
+            sb.hge[idx][1][i] = (float)(-0.5 * g1d * g1d * m);
+            sb.c[idx][i] = __ldg(prm.tg + (22 + i) * prm.tne + t);
+            sb.v[idx][i] = __ldg(prm.tel + 3 * t + i);
         }
         sb.n[idx] = make_float4((float)g.n[0], (float)g.n[1], (float)g.n[2], 0.f);
         sb.ie[idx] = g.ie;
@@ -509,32 +512,35 @@ __device__ __forceinline__ void regular_dp0_mixed_sym_tile(const RegParams &prm,
     double sc[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) sc[d] = __ldg(prm.sg + (22 + d) * prm.sne + s);
-    float2 yx[NP], yyy[NP], yz[NP], yy2[NP], wq2[NP];
-    const float sn0 = (float)gs.n[0], sn1 = (float)gs.n[1], sn2 = (float)gs.n[2];
+    float f[2][3];     // vertex offsets f_0, f_1 (f_2 = -f_0 - f_1)
+    float2 hgf[3];     // -g_q^2 |f_j|^2 / 2 of both orbits
+    {
+        double fd[3][3];
+        orbit_offsets(gs, fd);
 #pragma unroll
-    for (int j = 0; j < NP; ++j) {
-        float o[2][3];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            double v[3];
-            to_global(gs, rule.x[2 * j + h], rule.y[2 * j + h], v);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) o[h][d] = (float)(kap * (v[d] - sc[d]));
+        for (int j = 0; j < 3; ++j) {
+            const double m = -0.5 * kap * kap * odot(fd[j], fd[j]);
+            hgf[j] = f2((float)(g0d * g0d * m), (float)(g1d * g1d * m));
         }
-        yx[j] = f2(o[0][0], o[1][0]);
-        yyy[j] = f2(o[0][1], o[1][1]);
-        yz[j] = f2(o[0][2], o[1][2]);
-        yy2[j] = fma2(yz[j], yz[j], fma2(yyy[j], yyy[j], mul2(yx[j], yx[j])));
-        wq2[j] = f2(rule.wf[2 * j], rule.wf[2 * j + 1]);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            f[0][d] = (float)(kap * fd[0][d]);
+            f[1][d] = (float)(kap * fd[1][d]);
+        }
     }
+    const float sn0 = (float)gs.n[0], sn1 = (float)gs.n[1], sn2 = (float)gs.n[2];
     const double ek_r = (K == BEMPPCUDA_HELMHOLTZ_COMBINED) ? kap * prm.p[2] : kap;
     const double ek_i = (K == BEMPPCUDA_HELMHOLTZ_COMBINED) ? kap * prm.p[3] : 0.0;
     const double k2d = kap * kap;
-    // test-point weights: w_b for the second orbit, w_a / w_b applied in FP32 to the first
+    // weights: w_b for the second test orbit, w_a / w_b applied in FP32 to the first; the trial orbits' at the end
     const double wb = rule.w[NQ6 - 1];
     const float2 rho2 = b2((float)(rule.w[0] / wb));
+    const float wqa = rule.wf[0], wqb = rule.wf[NQ6 - 1];
     // centroid distances below near_r (scaled) may belong to vertex-sharing pairs
     const double near2 = prm.near_r > 0.0 ? (kap * prm.near_r) * (kap * prm.near_r) : 1e300;
+    const auto fdot = [](const float a[3], float b0, float b1, float b2_) {
+        return fmaf(a[2], b2_, fmaf(a[1], b1, a[0] * b0));
+    };
 
     for (int tt = 0; tt < tcount; ++tt) {
         const int64_t row = t0 + tt;
@@ -551,113 +557,131 @@ __device__ __forceinline__ void regular_dp0_mixed_sym_tile(const RegParams &prm,
             if (ST::helm) phase_reduced32(rc, &ph_s, &ph_c);
             // e^{-beta r_c'} (complex k), e^{-r_c'} (modified Helmholtz)
             const double amp = CK ? exp_neg_reduced(betd * rc) : (ST::modhelm ? exp_neg_reduced(rc) : 1.0);
-            const float D0f = (float)D0, D1f = (float)D1, D2f = (float)D2;
-            const float2 rcf2 = b2((float)rc), rc2f2 = b2((float)rc2);
-            // k (y - x).n_j = cp_p (y lies in the plane of j, so (y - c_j).n_j = 0) and
-            // k (x - y).n_i = ynt_q ((x - c_i).n_i = 0): one factor per test point, one per trial point
-            float nh0 = 0.f, nh1 = 0.f, nh2 = 0.f, Dn = 0.f;
-            float2 ynt[NP];
+            const float D0f = (float)D0, D1f = (float)D1, D2f = (float)D2, rcf = (float)rc;
+            const float2 rc_2 = b2(rcf), mrc_2 = b2(-rcf), mrc2_2 = b2(-(float)rc2);
+            // k (y - x).n_s = Dn - g_p e_i . n_s, one factor per test point; k (x - y).n_t = -Dt - g_q f_j . n_t,
+            // one per trial point
+            float Dn = 0.f;
+            float2 ynt[3];
             if (ST::dlp_part) {
                 const float4 tn = sb.n[tt];
-                const float2 Dt = b2(-fmaf(D2f, tn.z, fmaf(D1f, tn.y, D0f * tn.x)));
-#pragma unroll
-                for (int j = 0; j < NP; ++j)
-                    ynt[j] = fma2(yz[j], b2(-tn.z), fma2(yyy[j], b2(-tn.y), fma2(yx[j], b2(-tn.x), Dt)));
+                const float mDt = -fmaf(D2f, tn.z, fmaf(D1f, tn.y, D0f * tn.x));
+                const float m0 = -fdot(f[0], tn.x, tn.y, tn.z), m1 = -fdot(f[1], tn.x, tn.y, tn.z);
+                ynt[0] = fma2(b2(m0), g2, b2(mDt));
+                ynt[1] = fma2(b2(m1), g2, b2(mDt));
+                ynt[2] = fma2(b2(-(m0 + m1)), g2, b2(mDt));
                 Dn = fmaf(D2f, sn2, fmaf(D1f, sn1, D0f * sn0));
-                nh0 = 0.5f * sn0;
-                nh1 = 0.5f * sn1;
-                nh2 = 0.5f * sn2;
             }
-            const float2 D0d = b2(2.f * D0f), D1d = b2(2.f * D1f), D2d = b2(2.f * D2f);
-            float2 A[NP];
+            float2 hA[3];  // -A_q / 2
+            {
+                const float a0 = -fdot(f[0], D0f, D1f, D2f), a1 = -fdot(f[1], D0f, D1f, D2f);
+                hA[0] = fma2(b2(a0), g2, hgf[0]);
+                hA[1] = fma2(b2(a1), g2, hgf[1]);
+                hA[2] = fma2(b2(-(a0 + a1)), g2, hgf[2]);
+            }
+            float E[3][3], De[3], en[3];  // e_i . f_j, D . e_i, e_i . n_s
 #pragma unroll
-            for (int j = 0; j < NP; ++j) A[j] = fma2(D2d, yz[j], fma2(D1d, yyy[j], fma2(D0d, yx[j], yy2[j])));
-            float2 s0r = b2(0.f), s0i = b2(0.f), ur = b2(0.f), ui = b2(0.f), vr = b2(0.f), vi = b2(0.f);
+            for (int i = 0; i < 2; ++i) {
+                const float e0 = sb.e[tt][i][0], e1 = sb.e[tt][i][1], e2 = sb.e[tt][i][2];
+                De[i] = fmaf(D2f, e2, fmaf(D1f, e1, D0f * e0));
+                if (ST::dlp_part) en[i] = fmaf(sn2, e2, fmaf(sn1, e1, sn0 * e0));
+                E[i][0] = fdot(f[0], e0, e1, e2);
+                E[i][1] = fdot(f[1], e0, e1, e2);
+                E[i][2] = -(E[i][0] + E[i][1]);
+            }
+            De[2] = -(De[0] + De[1]);
+            if (ST::dlp_part) en[2] = -(en[0] + en[1]);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) E[2][j] = -(E[0][j] + E[1][j]);
+            float2 s0r = b2(0.f), s0m = b2(0.f), um = b2(0.f), ui = b2(0.f), vm = b2(0.f), vi = b2(0.f);
 #pragma unroll
             for (int p = 0; p < NQ6; ++p) {
+                const int i = p % 3, op = p / 3;
                 if (p == NQ6 / 2) {  // second orbit: the first orbit's sums times w_a / w_b
                     s0r = mul2(s0r, rho2);
-                    s0i = mul2(s0i, rho2);
-                    ur = mul2(ur, rho2);
+                    s0m = mul2(s0m, rho2);
+                    um = mul2(um, rho2);
                     ui = mul2(ui, rho2);
-                    vr = mul2(vr, rho2);
+                    vm = mul2(vm, rho2);
                     vi = mul2(vi, rho2);
                 }
-                const float4 mxy = sb.mxy[tt][p], mzw = sb.mzw[tt][p];
-                const float2 mx = f2(mxy.x, mxy.y), my = f2(mxy.z, mxy.w), mz = f2(mzw.x, mzw.y);
-                const float2 Bp2 = b2(fmaf(D2f, mzw.x, fmaf(D1f, mxy.z, fmaf(D0f, mxy.x, mzw.z))));
-                float2 cp2 = b2(0.f);
-                if (ST::dlp_part) cp2 = b2(fmaf(mzw.x, nh2, fmaf(mxy.z, nh1, fmaf(mxy.x, nh0, Dn))));
-                float2 pur = b2(0.f), pui = b2(0.f);  // sum over q of the A_ij double-layer factor, times cp per p
+                const float2 hB = b2(fmaf(go[op], De[i], sb.hge[tt][op][i]));  // -B_p / 2
+                const float2 gp2 = f2(go[op] * go[0], go[op] * go[1]);
+                const float2 cp2 = b2(ST::dlp_part ? fmaf(-go[op], en[i], Dn) : 0.f);
+                float2 pum = b2(0.f), pui = b2(0.f);  // sums over q of the A_ij double-layer factors, times cp per p
 #pragma unroll
-                for (int j = 0; j < NP; ++j) {
-                    const float2 sdot = fma2(yz[j], mz, fma2(yyy[j], my, fma2(yx[j], mx, add2(A[j], Bp2))));
-                    const float2 r2 = add2(rc2f2, sdot);
-                    const float2 rinv = f2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
-                    const float2 f = mul2(wq2[j], rinv);
+                for (int j = 0; j < 3; ++j) {
+                    const float2 hs = fma2(b2(E[i][j]), gp2, add2(hA[j], hB));  // -s / 2
+                    const float2 mr2 = fma2(hs, b2(2.f), mrc2_2);              // -r'^2
+                    const float2 rinv = f2(rsqrt_approx(-mr2.x), rsqrt_approx(-mr2.y));
+                    // -theta
+                    float2 mt = b2(0.f);
+                    if (ST::helm || ST::modhelm) {
+                        const float2 t = fma2(mr2, rinv, rc_2);
+                        mt = fma2(fma2(t, fma2(t, b2(0.5f), mrc_2), hs), rinv, t);
+                    }
                     if (!ST::helm) {
                         // modified Helmholtz: e^{-theta} per pair (e^{-r_c'} per element pair), the double
                         // layers' (1 + r') e^{-theta}
                         float2 am = b2(1.f), am1 = b2(1.f);
                         if (ST::modhelm) {
-                            const float2 den = fma2(r2, rinv, rcf2);
-                            const float2 th = mul2(sdot, f2(rcp_approx(den.x), rcp_approx(den.y)));
-                            am = f2(__expf(-th.x), __expf(-th.y));
-                            am1 = mul2(am, fma2(r2, rinv, b2(1.f)));
+                            am = f2(__expf(mt.x), __expf(mt.y));
+                            am1 = mul2(am, add2(b2(1.f), mul2(mul2(mr2, rinv), b2(-1.f))));
                         }
-                        if (ST::slp_part) s0r = ST::modhelm ? fma2(f, am, s0r) : add2(f, s0r);
+                        if (ST::slp_part) s0r = ST::modhelm ? fma2(rinv, am, s0r) : add2(rinv, s0r);
                         if (ST::dlp_part) {
-                            float2 fr = mul2(mul2(f, rinv), rinv);
+                            float2 fr = mul2(mul2(rinv, rinv), rinv);
                             if (ST::modhelm) fr = mul2(fr, am1);
-                            pur = add2(fr, pur);
-                            vr = fma2(fr, ynt[j], vr);
+                            pum = add2(fr, pum);
+                            vm = fma2(fr, ynt[j], vm);
                         }
                     } else {
-                        const float2 den = fma2(r2, rinv, rcf2);
-                        const float2 th = mul2(sdot, f2(rcp_approx(den.x), rcp_approx(den.y)));
-                        float2 sn, cs;
-                        sincos2_sym<PHC>(th, &sn, &cs);
+                        float2 ms, cs;  // -sin, cos of theta
+                        sincos2_sym<PHC>(mt, &ms, &cs);
                         if (CK) {
-                            const float2 am = f2(__expf(-bet2.x * th.x), __expf(-bet2.x * th.y));
+                            const float2 am = f2(__expf(bet2.x * mt.x), __expf(bet2.x * mt.y));
                             cs = mul2(cs, am);
-                            sn = mul2(sn, am);
+                            ms = mul2(ms, am);
                         }
                         if (ST::slp_part) {
-                            s0r = fma2(f, cs, s0r);
-                            s0i = fma2(f, sn, s0i);
+                            s0r = fma2(rinv, cs, s0r);
+                            s0m = fma2(rinv, ms, s0m);
                         }
                         if (ST::dlp_part) {
-                            const float2 fr = mul2(f, rinv);
+                            const float2 fr = mul2(rinv, rinv);
                             const float2 rb = CK ? add2(rinv, bet2) : rinv;  // 1 / r' (+ beta)
-                            const float2 h1 = fma2(rb, cs, sn);
-                            const float2 h2 = fma2(f2(-rb.x, -rb.y), sn, cs);
+                            const float2 mh1 = fma2(mul2(rb, b2(-1.f)), cs, ms);  // -h1
+                            const float2 h2 = fma2(rb, ms, cs);
                             const float2 gt = mul2(fr, ynt[j]);
-                            pur = fma2(fr, h1, pur);
+                            pum = fma2(fr, mh1, pum);
                             pui = fma2(fr, h2, pui);
-                            vr = fma2(gt, h1, vr);
+                            vm = fma2(gt, mh1, vm);
                             vi = fma2(gt, h2, vi);
                         }
                     }
                 }
                 if (ST::dlp_part) {
-                    ur = fma2(cp2, pur, ur);
+                    um = fma2(cp2, pum, um);
                     if (ST::helm) ui = fma2(cp2, pui, ui);
                 }
             }
-            // entry = w_b [kappa eta S0 + kappa^2 (-h1 sum + i h2 sum)], rotated by exp(i r_c') and scaled
+            // entry = w_b [kappa eta S0 + kappa^2 (-h1 sum + i h2 sum)], rotated by exp(i r_c') and scaled; um and vm
+            // hold the -h1 sums (Helmholtz) or the sums of w (d'.n) / r'^3 (real kernels)
+            const auto orbits = [&](float2 v) { return (double)fmaf(wqa, v.x, wqb * v.y); };
             double sr = 0.0, sim = 0.0;
             if (ST::slp_part) {
-                const double xr = (double)(s0r.x + s0r.y), xi = (double)(s0i.x + s0i.y);
+                const double xr = orbits(s0r), xi = ST::helm ? -orbits(s0m) : 0.0;
                 sr = fma(ek_r, xr, -ek_i * xi);
                 sim = fma(ek_r, xi, ek_i * xr);
             }
             double dr = 0.0, di = 0.0, er = 0.0, ei = 0.0;
             if (ST::dlp_part) {
-                dr = -k2d * (double)(ur.x + ur.y);
-                er = -k2d * (double)(vr.x + vr.y);
+                const double sg = ST::helm ? k2d : -k2d;
+                dr = sg * orbits(um);
+                er = sg * orbits(vm);
                 if (ST::helm) {
-                    di = k2d * (double)(ui.x + ui.y);
-                    ei = k2d * (double)(vi.x + vi.y);
+                    di = k2d * orbits(ui);
+                    ei = k2d * orbits(vi);
                 }
             }
             if (ST::swap) {

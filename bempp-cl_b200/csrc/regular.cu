@@ -417,8 +417,10 @@ int bc_regular_launch(const bemppcuda_regular_args *a, cudaStream_t st) {
             bc_set_error("kernel %d not valid for boundary assembly", a->kernel);
             return BEMPPCUDA_ERR_INVALID;
         }
-        err = launch_dp0_kernel(a->kernel, prm, rule, oc, sym_form(a->kernel, prm.p, a->phase_radius, orbits, orbit), mixed,
-                                phase_class, sym, row0, row1, st);
+        // (the mixed symmetric sweep is written for the two-orbit rule: any other 6-point rule runs in FP64)
+        const int form = sym_form(a->kernel, prm.p, a->phase_radius, orbits, orbit);
+        err = launch_dp0_kernel(a->kernel, prm, rule, oc, form, sym && !orbits ? 0 : mixed, phase_class, sym, row0,
+                                row1, st);
     } else if ((a->assembly == BEMPPCUDA_ASM_EFIE || a->assembly == BEMPPCUDA_ASM_MFIE) && a->nq == NQ6 &&
                (orbits || (!mixed && a->params[1] == 0.0)) && !a->overwrite &&
                a->kernel == BEMPPCUDA_HELMHOLTZ_SLP && (a->params[0] != 0.0 || a->params[1] != 0.0) &&

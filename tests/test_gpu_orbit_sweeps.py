@@ -4,7 +4,7 @@ p1_mixed.cuh), run on a B200.
 Offset classes 2, 1 and 0 with real and complex wavenumbers against the oracle; two sheets a thousandth of an element
 apart, whose distances the expanded square would lose (they are differenced); grids around the row blocks of
 one, of a few and of 32 rows; and the 6-point rule with its points in another order, which takes the points form or
-the general kernels (FP64 for a mixed P1 operator).  FP64 1e-12, mixed 1e-6 as the other tests; the nearly touching sheets 1e-10: the
+the general kernels (FP64 for a mixed operator).  FP64 1e-12, mixed 1e-6 as the other tests; the nearly touching sheets 1e-10: the
 sheets' coordinates differ in their last digits, eps / 1e-3 of the gap.
 """
 
@@ -104,8 +104,6 @@ def test_rule_in_another_order(case, interface, monkeypatch):
     from bempp_cuda import assembly
     from bempp_cuda.shapes import ellipsoid
 
-    if interface == "cuda_mixed" and case[2] == "DP":
-        pytest.skip("the mixed DP0 sweep is written for points in this order")
     grid = ellipsoid(2, 1.0, 0.8, 1.2)
     ref = _operator(*case, grid, 1.2)[0].weak_form().A
     pts, wts = assembly.regular_rule(4)
