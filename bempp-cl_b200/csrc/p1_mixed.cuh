@@ -5,14 +5,14 @@
 // the mixed DP0 kernels (dp0.cuh).
 //
 // Lengths are in units of 1/k.  Per element pair the centroid offset
-// D = k (c_s - c_t), r_c' = |D| and exp(i r_c') are FP64; per point pair only
-//   r'^2 - r_c'^2 = A_q + B_p + yo_q . m_p,
-//   A_q = |yo_q|^2 + 2 D . yo_q,  B_p = |xo_p|^2 - 2 D . xo_p,  m_p = -2 xo_p,
-// (xo, yo: the points' offsets from their centroids, times k) is formed in
-// FP32, 1/r' by rsqrt.approx, the phase offset theta = (r'^2 - r_c'^2) /
-// (r' + r_c') without cancellation and its sine / cosine by the fitted FP32
-// polynomials; trial points q, q+1 travel together through packed f32x2 FMAs.
-// Single layer: the trial sums T_j(p) = sum_q w_q psi_j(q) exp(i theta) / r'.
+// D = k (c_s - c_t), r_c' = |D| and exp(i r_c') are FP64; per point pair, with
+// the two-orbit rule (orbit.cuh; x_p = c_t + g_p e_i, y_q = c_s + g_q f_j),
+//   s = r'^2 - r_c'^2 = A_q + B_p - 2 g_p g_q e_i . f_j
+// is formed in FP32, 1/r' by rsqrt.approx, the phase offset theta = r' - r_c'
+// by one Newton step on theta^2 + 2 r_c' theta = s (dp0_sym.cuh) and its sine /
+// cosine by the fitted FP32 polynomials.  The trial points of one vertex, one
+// of each orbit, travel together through packed f32x2 FMAs; the blocks of the
+// trial sums T_j(p) = sum_q w_q psi_j(q) K add real and imaginary parts packed.
 // Double layers: with h = (i r' - 1) exp(i theta) / r'^3 and d' = k (y - x),
 // a quadrature point lies in its own element's plane, so
 //   d' . n_s = D . n_s - xo_p . n_s      (one value per test point)
@@ -68,7 +68,8 @@
 namespace bc {
 
 struct TestBlockP1m {
-    float4 m[P1_TCHUNK][NQ6];  // (-2 xo, |xo|^2), xo = k (x_p - c_t)
+    float e[P1_TCHUNK][3][3];    // vertex offsets kappa (v_i - c_t)
+    float hge[P1_TCHUNK][2][3];  // -g_o^2 |e_i|^2 / 2 per orbit
     double c[P1_TCHUNK][3];
     double n[P1_TCHUNK][3];
     double ie[P1_TCHUNK];
@@ -81,7 +82,7 @@ struct TestBlockP1m {
 // constant function takes the rule's weights in place of the P1 shape weights; scalar operators, no
 // symmetric sweep).
 template <int ASM, int K, int PHC, bool SYM, bool CK = false, int NT = 3, int NS = 3>
-__global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, QuadRule rule) {
+__global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, OrbitConsts oc) {
     constexpr bool LAP = K == BEMPPCUDA_LAPLACE_SLP || K == BEMPPCUDA_LAPLACE_DLP || K == BEMPPCUDA_LAPLACE_ADLP;
     constexpr bool MH = K == BEMPPCUDA_MODHELM_SLP || K == BEMPPCUDA_MODHELM_DLP || K == BEMPPCUDA_MODHELM_ADLP;
     constexpr bool REAL = LAP || MH;  // real kernel, real result
@@ -98,7 +99,8 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, Q
     constexpr bool SKEW = SYM && (DL || AD);
     constexpr bool NS_SUM = DL || SKEW;  // sums multiplied by d'.n_s per test point
     constexpr bool NT_SUM = AD || SKEW;  // sums with -d'.n_t per pair
-    constexpr int NP = NQ6 / 2;
+    // the FP32 sums hold the real and imaginary parts of the kernel up to these signs
+    constexpr double SGR = DL || AD || MFIE ? -1.0 : 1.0, SGI = -SGR;
     __shared__ TestBlockP1m sb;
     __shared__ double scurl[HYP || RWG ? P1_TCHUNK : 1][3][3];  // curls (HYP) or J_t, v0_t (RWG)
     __shared__ WarpColumns swc[DP0_THREADS / 32];
@@ -111,9 +113,8 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, Q
     const double betd = CK ? prm.p[1] / prm.p[0] : (MH ? 1.0 : 0.0);
     const float bet = (float)betd;
 
-    // test elements per CTA: P1_TCHUNK, and for the Maxwell operators ceil(ntest / gridDim.y) <= P1_TCHUNK
-    // (their launch picks 16 on small grids; a runtime height made the scalar kernels slower)
-    const int rows = RWG ? (int)((prm.ntest + gridDim.y - 1) / gridDim.y) : P1_TCHUNK;
+    // test elements per CTA: ceil(ntest / gridDim.y) <= P1_TCHUNK (the launch picks the row blocks)
+    const int rows = (int)((prm.ntest + gridDim.y - 1) / gridDim.y);
     const int64_t t0 = (int64_t)blockIdx.y * rows;
     if (SYM && t0 >= ((int64_t)blockIdx.x + 1) * DP0_THREADS) return;  // below the diagonal
     const int tcount = (int)min((int64_t)rows, prm.ntest - t0);
@@ -124,12 +125,15 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, Q
         double c[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) c[d] = __ldg(prm.tg + (22 + d) * prm.tne + t);
-        for (int p = 0; p < NQ6; ++p) {
-            double x[3];
-            to_global(g, rule.x[p], rule.y[p], x);
-            const float o0 = (float)(kap * (x[0] - c[0])), o1 = (float)(kap * (x[1] - c[1])),
-                        o2 = (float)(kap * (x[2] - c[2]));
-            sb.m[idx][p] = make_float4(-2.f * o0, -2.f * o1, -2.f * o2, fmaf(o2, o2, fmaf(o1, o1, o0 * o0)));
+        double eo[3][3];
+        orbit_offsets(g, eo);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) sb.e[idx][i][d] = (float)(kap * eo[i][d]);
+            const double m = -0.5 * kap * kap * odot(eo[i], eo[i]);
+            sb.hge[idx][0][i] = (float)(oc.gg[0] * m);
+            sb.hge[idx][1][i] = (float)(oc.gg[1] * m);
         }
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -172,23 +176,31 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, Q
     double sc[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) sc[d] = __ldg(prm.sg + (22 + d) * prm.sne + s);
-    // trial offsets k (y_q - c_s), q = 2 jj, 2 jj + 1 packed
-    float2 yx[NP], yyy[NP], yz[NP], yy2[NP];
+    // vertex offsets f_0, f_1 (f_2 = -f_0 - f_1) and -g_q^2 |f_j|^2 / 2 of both orbits
+    float f[2][3];
+    float2 hgf[3];
+    {
+        double fd[3][3];
+        orbit_offsets(gs, fd);
 #pragma unroll
-    for (int jj = 0; jj < NP; ++jj) {
-        float o[2][3];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            double v[3];
-            to_global(gs, rule.x[2 * jj + h], rule.y[2 * jj + h], v);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) o[h][d] = (float)(kap * (v[d] - sc[d]));
+        for (int j = 0; j < 3; ++j) {
+            const double m = -0.5 * kap * kap * odot(fd[j], fd[j]);
+            hgf[j] = f2((float)(oc.gg[0] * m), (float)(oc.gg[1] * m));
         }
-        yx[jj] = f2(o[0][0], o[1][0]);
-        yyy[jj] = f2(o[0][1], o[1][1]);
-        yz[jj] = f2(o[0][2], o[1][2]);
-        yy2[jj] = fma2(yz[jj], yz[jj], fma2(yyy[jj], yyy[jj], mul2(yx[jj], yx[jj])));
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            f[0][d] = (float)(kap * fd[0][d]);
+            f[1][d] = (float)(kap * fd[1][d]);
+        }
     }
+    // orbit constants in FP32: offsets g, and w times the linear functions at a point: the own vertex's (c + d) and
+    // the other two's (d).  (c and d times the orbit's sum, as in FP64, would cancel: c < 0 in the first orbit.)
+    const float go[2] = {(float)oc.g[0], (float)oc.g[1]};
+    const float2 g2 = f2(go[0], go[1]);
+    const float2 own2 = f2((float)(oc.c[0] + oc.d[0]), (float)(oc.c[1] + oc.d[1])), oth2 = f2((float)oc.d[0], (float)oc.d[1]);
+    const float2 w2 = f2((float)oc.w[0], (float)oc.w[1]);
+    const float own_[2] = {own2.x, own2.y}, oth_[2] = {oth2.x, oth2.y}, wp_[2] = {w2.x, w2.y};
+    const auto fdot = [](const float a[3], float x, float y, float z) { return fmaf(a[2], z, fmaf(a[1], y, a[0] * x)); };
     const float sn0 = (float)gs.n[0], sn1 = (float)gs.n[1], sn2 = (float)gs.n[2];
     double curl_s[3][3];
     if (HYP) surface_curls(prm.sg, prm.sne, s, gs.n, curl_s);
@@ -242,115 +254,147 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, Q
             }
         }
         const float D0f = (float)D0, D1f = (float)D1, D2f = (float)D2;
-        const float2 rcf2 = b2((float)rc), rc2f2 = b2((float)rc2);
-        const float2 D0d = b2(2.f * D0f), D1d = b2(2.f * D1f), D2d = b2(2.f * D2f);
-        float2 A[NP];
-#pragma unroll
-        for (int jj = 0; jj < NP; ++jj) A[jj] = fma2(D2d, yz[jj], fma2(D1d, yyy[jj], fma2(D0d, yx[jj], yy2[jj])));
-        // normal terms: D . n_s; -(d'.n_t) = -(D . n_t) - yo_q . n_t per trial point
-        const float tn0 = (float)sb.n[tt][0], tn1 = (float)sb.n[tt][1], tn2 = (float)sb.n[tt][2];
-        const float Dns = fmaf(D2f, sn2, fmaf(D1f, sn1, D0f * sn0));
-        float2 mdt[NP];
-        if (NT_SUM) {
-            const float2 mDnt = b2(-fmaf(D2f, tn2, fmaf(D1f, tn1, D0f * tn0)));
-#pragma unroll
-            for (int jj = 0; jj < NP; ++jj)
-                mdt[jj] = fma2(yz[jj], b2(-tn2), fma2(yyy[jj], b2(-tn1), fma2(yx[jj], b2(-tn0), mDnt)));
+        const float rcf = (float)rc;
+        const float2 rc_2 = b2(rcf), mrc_2 = b2(-rcf), mrc2_2 = b2(-(float)rc2);
+        float2 hA[3];  // -A_q / 2
+        {
+            const float a0 = -fdot(f[0], D0f, D1f, D2f), a1 = -fdot(f[1], D0f, D1f, D2f);
+            hA[0] = fma2(b2(a0), g2, hgf[0]);
+            hA[1] = fma2(b2(a1), g2, hgf[1]);
+            hA[2] = fma2(b2(-(a0 + a1)), g2, hgf[2]);
         }
-        float lre[3][3], lim[3][3];              // block of (i, j): single layer, or the first double layer
-        float ure[3][3], uim[3][3];              // SKEW: the transposed pair's block
+        // normal terms: D . n_s; -(d'.n_t) = -(D . n_t) - g_q f_j . n_t per trial point
+        const float Dns = NS_SUM ? fmaf(D2f, sn2, fmaf(D1f, sn1, D0f * sn0)) : 0.f;
+        float2 cm[3] = {b2(0.f), b2(0.f), b2(0.f)};
+        if (NT_SUM) {
+            const float tn0 = (float)sb.n[tt][0], tn1 = (float)sb.n[tt][1], tn2 = (float)sb.n[tt][2];
+            const float2 mDt = b2(-fmaf(D2f, tn2, fmaf(D1f, tn1, D0f * tn0)));
+            const float m0 = -fdot(f[0], tn0, tn1, tn2), m1 = -fdot(f[1], tn0, tn1, tn2);
+            cm[0] = fma2(b2(m0), g2, mDt);
+            cm[1] = fma2(b2(m1), g2, mDt);
+            cm[2] = fma2(b2(-(m0 + m1)), g2, mDt);
+        }
+        float E[3][3], De[3], en[3] = {0.f, 0.f, 0.f};  // e_i . f_j, D . e_i, e_i . n_s
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
+        for (int i = 0; i < 2; ++i) {
+            const float e0 = sb.e[tt][i][0], e1 = sb.e[tt][i][1], e2 = sb.e[tt][i][2];
+            De[i] = fmaf(D2f, e2, fmaf(D1f, e1, D0f * e0));
+            if (NS_SUM) en[i] = fmaf(sn2, e2, fmaf(sn1, e1, sn0 * e0));
+            E[i][0] = fdot(f[0], e0, e1, e2);
+            E[i][1] = fdot(f[1], e0, e1, e2);
+            E[i][2] = -(E[i][0] + E[i][1]);
+        }
+        De[2] = -(De[0] + De[1]);
+        if (NS_SUM) en[2] = -(en[0] + en[1]);
 #pragma unroll
-            for (int j = 0; j < 3; ++j) lre[i][j] = lim[i][j] = ure[i][j] = uim[i][j] = 0.f;
-#pragma unroll 2
+        for (int j = 0; j < 3; ++j) E[2][j] = -(E[0][j] + E[1][j]);
+        // (re, im) blocks: the block of (i, j): single layer, or its double layer; SKEW: the transposed pair's
+        float2 l[NT][NS], u[SKEW ? NT : 1][SKEW ? NS : 1];
+        const auto axpy = [](float a, float2 x, float2 y) -> float2 {
+            return REAL ? f2(fmaf(a, x.x, y.x), 0.f) : fma2(b2(a), x, y);
+        };
+#pragma unroll
         for (int p = 0; p < NQ6; ++p) {
-            const float4 m = sb.m[tt][p];
-            const float Bp = fmaf(D2f, m.z, fmaf(D1f, m.y, fmaf(D0f, m.x, m.w)));
-            const float2 mx = b2(m.x), my = b2(m.y), mz = b2(m.z), Bp2 = b2(Bp);
-            // d'.n_s at this test point: D . n_s - xo . n_s = D . n_s + (m . n_s) / 2
-            const float dns = NS_SUM ? fmaf(0.5f, fmaf(m.z, sn2, fmaf(m.y, sn1, m.x * sn0)), Dns) : 0.f;
-            float2 tre[3] = {b2(0.f), b2(0.f), b2(0.f)}, tim[3] = {b2(0.f), b2(0.f), b2(0.f)};
-            float2 vre[3] = {b2(0.f), b2(0.f), b2(0.f)}, vim[3] = {b2(0.f), b2(0.f), b2(0.f)};
+            const int i = p % 3, op = p / 3;
+            const float2 hB = b2(fmaf(go[op], De[i], sb.hge[tt][op][i]));  // -B_p / 2
+            const float2 gp2 = f2(go[op] * go[0], go[op] * go[1]);
+            float2 kr[3], ki[3];
 #pragma unroll
-            for (int jj = 0; jj < NP; ++jj) {
-                const float2 sdot = fma2(yz[jj], mz, fma2(yyy[jj], my, fma2(yx[jj], mx, add2(A[jj], Bp2))));
-                const float2 r2 = add2(rc2f2, sdot);
-                const float2 rinv = f2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
-                // cs + i sn: exp(i theta) (Helmholtz), times exp(-beta theta) (complex k); exp(-theta)
-                // (modified, sn = 0); 1 (Laplace)
-                float2 sn = b2(0.f), cs = b2(1.f);
+            for (int j = 0; j < 3; ++j) {
+                const float2 hs = fma2(b2(E[i][j]), gp2, add2(hA[j], hB));  // -s / 2
+                const float2 mr2 = fma2(hs, b2(2.f), mrc2_2);              // -r'^2
+                const float2 rinv = f2(rsqrt_approx(-mr2.x), rsqrt_approx(-mr2.y));
+                const float2 mrp = mul2(mr2, rinv);  // -r'
+                // cs - i ms: exp(i theta) (Helmholtz), times exp(-beta theta) (complex k); exp(-theta)
+                // (modified, ms = 0); 1 (Laplace)
+                float2 ms = b2(0.f), cs = b2(1.f);
                 if (!LAP) {
-                    const float2 den = fma2(r2, rinv, rcf2);
-                    const float2 th = mul2(sdot, f2(rcp_approx(den.x), rcp_approx(den.y)));
-                    if (!MH) sincos2<PHC>(th, &sn, &cs);
+                    const float2 t = fma2(mr2, rinv, rc_2);
+                    const float2 mt = fma2(fma2(t, fma2(t, b2(0.5f), mrc_2), hs), rinv, t);  // -theta
+                    if (!MH) sincos2<PHC>(mt, &ms, &cs);
                     if (MH || CK) {
-                        const float2 am = f2(__expf(-bet * th.x), __expf(-bet * th.y));
+                        const float2 am = f2(__expf(bet * mt.x), __expf(bet * mt.y));
                         cs = mul2(cs, am);
-                        if (CK) sn = mul2(sn, am);
+                        if (CK) ms = mul2(ms, am);
                     }
                 }
-                float2 kr, ki = b2(0.f);
+                ki[j] = b2(0.f);
                 if (!DL && !AD && !MFIE) {
-                    kr = mul2(rinv, cs);
-                    if (!REAL) ki = mul2(rinv, sn);
-                } else if (LAP) {
-                    kr = mul2(rinv, mul2(rinv, mul2(rinv, b2(-1.f))));  // -1 / r'^3
+                    kr[j] = mul2(rinv, cs);
+                    if (!REAL) ki[j] = mul2(rinv, ms);
                 } else {
-                    // h = (i k r - 1) e^{ikr} / r^3 in units of 1/kappa: ((-a cs - r' sn) + i (r' cs - a sn)) / r'^3,
-                    // a = 1 + beta r' (a = 1 for real k); modified: -(1 + r') e^{-r'} / r'^3
-                    const float2 rp = mul2(r2, rinv), r3 = mul2(rinv, mul2(rinv, rinv));
-                    if (MH) {
-                        kr = mul2(mul2(r3, cs), mul2(add2(rp, b2(1.f)), b2(-1.f)));
-                    } else if (CK) {
-                        const float2 a = fma2(b2(bet), rp, b2(1.f));
-                        kr = mul2(r3, mul2(fma2(rp, sn, mul2(a, cs)), b2(-1.f)));
-                        ki = mul2(r3, fma2(rp, cs, mul2(mul2(a, sn), b2(-1.f))));
+                    // -Re and Im of (ikr - 1) e^{ikr} / r^3 in units of 1/kappa: (a cs + r' sn, r' cs - a sn) / r'^3,
+                    // a = 1 + beta r' (a = 1 for real k); modified: (1 + r') e^{-r'} / r'^3
+                    const float2 r3 = mul2(rinv, mul2(rinv, rinv));
+                    if (LAP) {
+                        kr[j] = r3;
+                    } else if (MH) {
+                        kr[j] = mul2(mul2(r3, cs), fma2(mrp, b2(-1.f), b2(1.f)));
                     } else {
-                        kr = mul2(r3, mul2(fma2(rp, sn, cs), b2(-1.f)));
-                        ki = mul2(r3, fma2(rp, cs, mul2(sn, b2(-1.f))));
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < NS; ++j) {
-                    const float2 w = NS == 3 ? f2(rule.swf[2 * jj][j], rule.swf[2 * jj + 1][j])
-                                             : f2(rule.wf[2 * jj], rule.wf[2 * jj + 1]);
-                    if (!AD || SKEW) {  // plain sums (single layer; double layer: times d'.n_s below)
-                        tre[j] = fma2(kr, w, tre[j]);
-                        if (!REAL) tim[j] = fma2(ki, w, tim[j]);
-                    }
-                    if (NT_SUM) {  // sums with -(d'.n_t)
-                        const float2 wd = mul2(w, mdt[jj]);
-                        vre[j] = fma2(kr, wd, vre[j]);
-                        if (!REAL) vim[j] = fma2(ki, wd, vim[j]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < NT; ++i) {
-                const float ph = NT == 3 ? rule.swf[p][i] : rule.wf[p];
-                const float phs = NS_SUM ? ph * dns : ph;
-#pragma unroll
-                for (int j = 0; j < NS; ++j) {
-                    if (!DL && !AD) {
-                        lre[i][j] = fmaf(ph, tre[j].x + tre[j].y, lre[i][j]);
-                        if (!REAL) lim[i][j] = fmaf(ph, tim[j].x + tim[j].y, lim[i][j]);
-                    } else {
-                        // (i, j): double layer -> n_s sums, adjoint -> n_t sums; SKEW: the other one at (j, i)
-                        const float2 first_r = DL ? tre[j] : vre[j], first_i = DL ? tim[j] : vim[j];
-                        const float f1 = DL ? phs : ph;
-                        lre[i][j] = fmaf(f1, first_r.x + first_r.y, lre[i][j]);
-                        if (!REAL) lim[i][j] = fmaf(f1, first_i.x + first_i.y, lim[i][j]);
-                        if (SKEW) {
-                            const float2 sec_r = DL ? vre[j] : tre[j], sec_i = DL ? vim[j] : tim[j];
-                            const float f2_ = DL ? ph : phs;
-                            ure[i][j] = fmaf(f2_, sec_r.x + sec_r.y, ure[i][j]);
-                            if (!REAL) uim[i][j] = fmaf(f2_, sec_i.x + sec_i.y, uim[i][j]);
+                        const float2 rp = mul2(mrp, b2(-1.f));
+                        if (CK) {
+                            const float2 a = fma2(b2(bet), rp, b2(1.f));
+                            kr[j] = mul2(r3, fma2(mrp, ms, mul2(a, cs)));
+                            ki[j] = mul2(r3, fma2(rp, cs, mul2(a, ms)));
+                        } else {
+                            kr[j] = mul2(r3, fma2(mrp, ms, cs));
+                            ki[j] = mul2(r3, fma2(rp, cs, ms));
                         }
                     }
                 }
             }
+            // the trial sums of each test point: T_j (plain) and V_j (with -(d'.n_t))
+            const auto sums = [&](const float2 *k, int j) -> float {
+                float2 v;
+                if (NS == 3)
+                    v = fma2(k[j], own2, mul2(add2(k[(j + 1) % 3], k[(j + 2) % 3]), oth2));
+                else
+                    v = mul2(add2(add2(k[0], k[1]), k[2]), w2);
+                return v.x + v.y;
+            };
+            float2 T[NS], V[NS];
+            if (!AD || SKEW)
+#pragma unroll
+                for (int j = 0; j < NS; ++j) T[j] = f2(sums(kr, j), REAL ? 0.f : sums(ki, j));
+            if (NT_SUM) {
+                float2 vr[3], vi[3];
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    vr[j] = mul2(kr[j], cm[j]);
+                    vi[j] = REAL ? b2(0.f) : mul2(ki[j], cm[j]);
+                }
+#pragma unroll
+                for (int j = 0; j < NS; ++j) V[j] = f2(sums(vr, j), REAL ? 0.f : sums(vi, j));
+            }
+            // into the blocks: (i, j) double layer -> T times d'.n_s, adjoint -> V; SKEW: the other one at (j, i)
+            const float dns = NS_SUM ? fmaf(-go[op], en[i], Dns) : 1.f;
+#pragma unroll
+            for (int a = 0; a < NT; ++a) {
+                const float w = NT == 1 ? wp_[op] : a == i ? own_[op] : oth_[op], wn = NS_SUM ? w * dns : w;
+#pragma unroll
+                for (int j = 0; j < NS; ++j) {
+                    l[a][j] = axpy(DL ? wn : w, AD ? V[j] : T[j], p == 0 ? b2(0.f) : l[a][j]);
+                    if (SKEW) {
+                        constexpr int A_ = SKEW ? NT : 1, B_ = SKEW ? NS : 1;
+                        u[a % A_][j % B_] = axpy(DL ? w : wn, DL ? V[j] : T[j], p == 0 ? b2(0.f) : u[a % A_][j % B_]);
+                    }
+                }
+            }
         }
+        float lre[3][3], lim[3][3], ure[3][3], uim[3][3];
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+#pragma unroll
+            for (int j = 0; j < NS; ++j) {
+                const float2 v = l[i][j];
+                lre[i][j] = v.x;
+                lim[i][j] = v.y;
+                if (SKEW) {
+                    const float2 w = u[i % (SKEW ? NT : 1)][j % (SKEW ? NS : 1)];
+                    ure[i][j] = w.x;
+                    uim[i][j] = w.y;
+                }
+            }
         // k / (4 pi) or k^2 / (4 pi), |J_t| |J_s| exp(i r_c'), then the hypersingular combination;
         // EFIE: the moments, k (4 pi G = k e^{i theta} / r' in these units) and 1 / (4 pi), no |J|
         double ere[3][3], eim[3][3];
@@ -362,7 +406,7 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, Q
             for (int i = 0; i < 3; ++i)
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
-                    const double lr = kap * (double)lre[i][j], li = kap * (double)lim[i][j];
+                    const double lr = SGR * kap * (double)lre[i][j], li = SGI * kap * (double)lim[i][j];
                     rs[i] += lr;
                     is[i] += li;
                     cs_[j] += lr;
@@ -378,8 +422,8 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, Q
                 mim[0][a] = ci_[a];
 #pragma unroll
                 for (int b = 1; b < 3; ++b) {
-                    mre[a][b] = kap * (double)lre[a][b];
-                    mim[a][b] = kap * (double)lim[a][b];
+                    mre[a][b] = SGR * kap * (double)lre[a][b];
+                    mim[a][b] = SGI * kap * (double)lim[a][b];
                 }
             }
             efie_block<CK>(mre, mim, scurl[tt][0], scurl[tt][1], gs.j0, gs.j1, kap, CK ? prm.p[1] : 0.0, ere, eim);
@@ -393,7 +437,7 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, Q
             for (int i = 0; i < 3; ++i)
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
-                    const double lr = k3 * (double)lre[i][j], li = k3 * (double)lim[i][j];
+                    const double lr = SGR * k3 * (double)lre[i][j], li = SGI * k3 * (double)lim[i][j];
                     rs[i] += lr;
                     is[i] += li;
                     cs_[j] += lr;
@@ -422,8 +466,8 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, Q
             for (int i = 0; i < 3; ++i)
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
-                    sre += (double)lre[i][j];
-                    sim += (double)lim[i][j];
+                    sre += SGR * (double)lre[i][j];
+                    sim += SGI * (double)lim[i][j];
                 }
             // -k^2 (n_t . n_s), complex for a complex wavenumber; +w^2 (n_t . n_s) modified; 0 Laplace
             const double nn = sb.n[tt][0] * gs.n[0] + sb.n[tt][1] * gs.n[1] + sb.n[tt][2] * gs.n[2];
@@ -447,7 +491,7 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, Q
                     if (SKEW) st_t[i][pos[j]] = make_double2(0.0, 0.0);
                     continue;
                 }
-                double vr = RWG ? ere[i][j] : (double)lre[i][j], vi = RWG ? eim[i][j] : (double)lim[i][j];
+                double vr = RWG ? ere[i][j] : SGR * (double)lre[i][j], vi = RWG ? eim[i][j] : SGI * (double)lim[i][j];
                 if (HYP) {
                     const double cij = scurl[tt][i][0] * curl_s[j][0] + scurl[tt][i][1] * curl_s[j][1] +
                                        scurl[tt][i][2] * curl_s[j][2];
@@ -460,7 +504,7 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, Q
                 vr = tr;
                 double wr = vr, wi = vi;  // the (j, i) block: the same, or (SKEW) its own sums
                 if (SKEW) {
-                    const double ur = (double)ure[i][j], ui = (double)uim[i][j];
+                    const double ur = SGR * (double)ure[i][j], ui = SGI * (double)uim[i][j];
                     wr = ur * ph_c - ui * ph_s;
                     wi = fma(ur, ph_s, ui * ph_c);
                 }
@@ -484,28 +528,34 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, Q
                 atomicAdd(m + 2 * (r * ld + c) + 1, im);
             }
         };
+        // the rows of a column are summed together: one walk over its staging positions
+        for (int c = (int)lane; c < ncols; c += 32) {
+            const int b = wc.start[c], e = wc.start[c + 1];
+            double ar[NT], ai[NT], br[NT], bi[NT];
 #pragma unroll
-        for (int i = 0; i < NT; ++i) {
-            const int64_t row = sb.row[tt][i];
-            for (int c = (int)lane; c < ncols; c += 32) {
-                const int b = wc.start[c], e = wc.start[c + 1];
-                double ar = 0.0, ai = 0.0, br = 0.0, bi = 0.0;
-                for (int k = b; k < e; ++k) {
+            for (int i = 0; i < NT; ++i) ar[i] = ai[i] = br[i] = bi[i] = 0.0;
+            for (int k = b; k < e; ++k) {
+#pragma unroll
+                for (int i = 0; i < NT; ++i) {
                     const double2 v = st[i][k];
-                    ar += v.x;
-                    ai += v.y;
+                    ar[i] += v.x;
+                    if (!REAL) ai[i] += v.y;
                     if (SKEW) {
                         const double2 w = st_t[i][k];
-                        br += w.x;
-                        bi += w.y;
+                        br[i] += w.x;
+                        if (!REAL) bi[i] += w.y;
                     }
                 }
-                const int64_t col = wc.col[c];
-                if (ar != 0.0 || ai != 0.0) {
-                    add_entry(res, prm.ld, row, col, ar, ai);
-                    if (SYM && !SKEW && !prm.defer_transpose) add_entry(res, prm.ld, col, row, ar, ai);
+            }
+            const int64_t col = wc.col[c];
+#pragma unroll
+            for (int i = 0; i < NT; ++i) {
+                const int64_t row = sb.row[tt][i];
+                if (ar[i] != 0.0 || ai[i] != 0.0) {
+                    add_entry(res, prm.ld, row, col, ar[i], ai[i]);
+                    if (SYM && !SKEW && !prm.defer_transpose) add_entry(res, prm.ld, col, row, ar[i], ai[i]);
                 }
-                if (SKEW && (br != 0.0 || bi != 0.0)) add_entry(res, prm.ld, col, row, br, bi);
+                if (SKEW && (br[i] != 0.0 || bi[i] != 0.0)) add_entry(res, prm.ld, col, row, br[i], bi[i]);
             }
         }
         __syncwarp();  // the staging arrays are rewritten by the next test element

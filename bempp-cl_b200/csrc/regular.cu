@@ -432,7 +432,7 @@ int bc_regular_launch(const bemppcuda_regular_args *a, cudaStream_t st) {
                           a->test.nsupport == a->trial.nsupport && a->test_grid.geom == a->trial_grid.geom &&
                           prm.ntest == prm.ntrial;
         if (mixed && rwg_mixed)
-            err = launch_p1_mixed_kernel(a->assembly, a->kernel, prm, rule, phase_class, rsym, st);
+            err = launch_p1_mixed_kernel(a->assembly, a->kernel, prm, oc, phase_class, rsym, st);
         else
             err = launch_rwg_kernel(a->assembly, prm, rule, oc, cls, rsym, st);
     } else if (const bool psym = !a->no_symmetry && a->grids_identical && a->test.support == a->trial.support &&
@@ -454,7 +454,7 @@ int bc_regular_launch(const bemppcuda_regular_args *a, cudaStream_t st) {
                             a->kernel == BEMPPCUDA_HELMHOLTZ_SLP || a->kernel == BEMPPCUDA_MODHELM_SLP);
         prm.defer_transpose = defer ? 1 : 0;
         if (mixed && p1_mixed)
-            err = launch_p1_mixed_kernel(a->assembly, a->kernel, prm, rule, phase_class, psym, st);
+            err = launch_p1_mixed_kernel(a->assembly, a->kernel, prm, oc, phase_class, psym, st);
         else
             err = launch_p1_kernel(a->assembly, a->kernel, prm, rule, oc, cls, psym, st);
         if (defer && err == cudaSuccess) err = launch_add_transpose(prm.result, a->test.ndofs, prm.ld, prm.is_complex, st);

@@ -30,7 +30,7 @@ cudaError_t launch_p1_kernel(int assembly, int kernel, const RegParams &prm, con
                              int cls, bool sym, cudaStream_t st);
 
 // The same in mixed precision, and the mixed Maxwell fields (regular_p1_mixed.cu).
-cudaError_t launch_p1_mixed_kernel(int assembly, int kernel, const RegParams &prm, const QuadRule &rule,
+cudaError_t launch_p1_mixed_kernel(int assembly, int kernel, const RegParams &prm, const OrbitConsts &oc,
                                    int phase_class, bool sym, cudaStream_t st);
 
 // Maxwell electric / magnetic fields in FP64 (regular_rwg.cu): any 6-point rule for a real wavenumber, the two-orbit
