@@ -62,9 +62,7 @@ def kernel_params(options):
 
 
 def _set_params(args, options):
-    p = kernel_params(options)
-    for i in range(4):
-        args.params[i] = float(p[i])
+    args.params[:] = kernel_params(options).tolist()
 
 
 def regular_rule(order):
@@ -119,12 +117,13 @@ def regular_into(
     kernel, assembly = kernel_ids(descriptor)
     if result.numel() == 0:
         return result  # a space without dofs: nothing to assemble
-    tgrid = geometry or device_grid(dual_to_range.grid)
-    sgrid = geometry or device_grid(domain.grid)
-    sspace = device_space(domain)
+    dev = _torch.cuda.current_device()
+    tgrid = geometry or device_grid(dual_to_range.grid, dev)
+    sgrid = geometry or device_grid(domain.grid, dev)
+    sspace = device_space(domain, dev)
     # an equal dual space shares the domain's device copy, which lets the
     # library take the symmetric sweep (it compares the pointers)
-    tspace = sspace if same_space(domain, dual_to_range) else device_space(dual_to_range)
+    tspace = sspace if same_space(domain, dual_to_range) else device_space(dual_to_range, dev)
     points, weights = regular_rule(parameters.quadrature.regular)
     args = _lib.RegularArgs()
     args.kernel = kernel
@@ -140,7 +139,7 @@ def regular_into(
     args.nq = len(weights)
     args.quad_points = points.ctypes.data
     args.quad_weights = weights.ctypes.data
-    args.result = ptr(result)
+    args.result = result.data_ptr()
     args.ld = result.stride(0)
     args.overwrite = 1 if overwrite else 0
     args.no_symmetry = 0 if symmetric else 1
@@ -290,26 +289,28 @@ def singular_into_dense(result, descriptor, domain, dual_to_range, parameters, d
     kernel, assembly = kernel_ids(descriptor)
     if result.numel() == 0:
         return result
+    dev = _torch.cuda.current_device()
     grid = domain.grid
-    rule = device_singular_rule(grid, parameters.quadrature.singular, dual_to_range.support, domain.support)
+    dgrid = geometry or device_grid(grid, dev)
+    rule = device_singular_rule(grid, parameters.quadrature.singular, dual_to_range.support, domain.support, dev)
     args = _lib.SingularArgs()
     args.kernel = kernel
     args.assembly = assembly
     args.is_complex = 1 if result.is_complex() else 0
     _set_params(args, descriptor.options)
-    args.grid = (geometry or device_grid(grid)).record()
-    args.test = device_space(dual_to_range).record()
-    args.trial = device_space(domain).record()
+    args.grid = dgrid.record()
+    args.test = device_space(dual_to_range, dev).record()
+    args.trial = device_space(domain, dev).record()
     if rows is None:
         rule.fill(args)
     else:
         sup = _np.asarray(dual_to_range.support_elements)
         rule.fill(args, rule.pair_range(int(sup[rows[0]]), int(sup[rows[1] - 1])))
     args.values = None
-    args.dense = ptr(result)
+    args.dense = result.data_ptr()
     args.ld = result.stride(0)
     args.diag_shift = float(diag_shift)
-    args.phase_radius = 1.0001 * 2.0 * (geometry or device_grid(grid)).radius
+    args.phase_radius = 1.0001 * 2.0 * dgrid.radius
     order = int(parameters.quadrature.singular)
     if mirror and (same_space(domain, dual_to_range) or _same_maps(domain, dual_to_range, assembly)):
         # every pair is listed in both orders and the vertex-adjacent rule (its weights follow the

@@ -25,14 +25,19 @@ from .quadrature import SingularPairs
 _CACHE_ATTR = "_bempp_cuda_device_cache"
 
 
+# A small operator's call is bound by the host (128 elements: 18 us on the device), so what a call looks up here is kept
+# short: one device lookup per call handed on as ``dev``, records built with the device copies that they point into,
+# the raw stream handle without a Stream object, no availability query once CUDA is initialised.
+
+
 def require_cuda():
-    if not _torch.cuda.is_available():
+    if not (_torch.cuda.is_initialized() or _torch.cuda.is_available()):
         raise RuntimeError("bempp_cuda needs a CUDA device (B200, sm_100a); none is visible")
     _lib.load()
 
 
 def current_stream():
-    return _ct.c_void_p(_torch.cuda.current_stream().cuda_stream)
+    return _ct.c_void_p(_torch._C._cuda_getCurrentRawStream(_torch.cuda.current_device()))
 
 
 def ptr(t):
@@ -115,9 +120,10 @@ class DeviceGrid(object):
         corners = vertices[elements]  # (ne, 3, 3)
         centroids = corners.mean(axis=1, keepdims=True)
         self.radius = float(_np.sqrt(((corners - centroids) ** 2).sum(axis=2)).max()) if self.nelements else 0.0
+        self._record = _lib.GridRec(self.nvertices, self.nelements, ptr(self.geom), ptr(self.elements))
 
     def record(self):
-        return _lib.GridRec(self.nvertices, self.nelements, ptr(self.geom), ptr(self.elements))
+        return self._record
 
 
 def _shared_on_grid(grid, name, array, dtype):
@@ -148,9 +154,7 @@ class DeviceSpace(object):
         self.mult = _shared_on_grid(grid, "mult", h["mult"], _torch.float64)
         self.normal_mult = _shared_on_grid(grid, "normal_mult", h["normal_mult"], _torch.int32)
         self.h2d_bytes = sum(h[name].nbytes for name in ("support", "l2g", "mult", "normal_mult"))
-
-    def record(self):
-        return _lib.Space(
+        self._record = _lib.Space(
             self.shapeset,
             self.nshape,
             self.nsupport,
@@ -162,6 +166,9 @@ class DeviceSpace(object):
             self.dof_is_position,
             0,
         )
+
+    def record(self):
+        return self._record
 
 
 class DeviceSingularRule(object):
@@ -183,6 +190,9 @@ class DeviceSingularRule(object):
         self.h2d_bytes = tp.nbytes + sp.nbytes + 8 * len(w) + sum(a.nbytes for a in ints)
         self._host_ints = ints
         self._by_test = None
+        self._tables = tuple(t.data_ptr() for t in (self.test_points, self.trial_points, self.weights))
+        self._pairs = tuple(t.data_ptr() for t in (self.test_elements, self.trial_elements, self.test_offsets,
+                                                   self.trial_offsets, self.weights_offsets, self.npoints))
 
     def by_test(self):
         """The pair arrays in test-element order (stable) on the device, and the sorted test elements (host)."""
@@ -201,25 +211,23 @@ class DeviceSingularRule(object):
     def fill(self, args, pairs=None):
         """Point the singular arguments at all pairs, or at pairs [begin, end) of the test-element order."""
         args.npoints_table = self.npoints_table
-        args.test_points = ptr(self.test_points)
-        args.trial_points = ptr(self.trial_points)
-        args.weights = ptr(self.weights)
+        args.test_points, args.trial_points, args.weights = self._tables
         args.nweights = self.nweights
         if pairs is None:
             args.npairs = self.npairs
-            arrays = (self.test_elements, self.trial_elements, self.test_offsets, self.trial_offsets,
-                      self.weights_offsets, self.npoints)
-            begin = 0
+            pointers = self._pairs
         else:
             begin, end = pairs
             args.npairs = max(0, end - begin)
-            arrays = self.by_test()[0]
+            pointers = [a.data_ptr() + 4 * begin for a in self.by_test()[0]]
         (args.test_elements, args.trial_elements, args.test_offsets, args.trial_offsets, args.weights_offsets,
-         args.npoints) = [_ct.c_void_p(a.data_ptr() + 4 * begin) for a in arrays]
+         args.npoints) = pointers
 
 
-def device_grid(grid):
-    dev = _torch.cuda.current_device()
+def device_grid(grid, dev=None):
+    """The device copy of ``grid`` on the current device (``dev``, where the caller has its index)."""
+    if dev is None:
+        dev = _torch.cuda.current_device()
     cache = _cache(grid)
     key = ("grid", dev)
     if key not in cache:
@@ -227,8 +235,10 @@ def device_grid(grid):
     return cache[key]
 
 
-def device_space(space):
-    dev = _torch.cuda.current_device()
+def device_space(space, dev=None):
+    """The device copy of ``space`` on the current device (``dev``, where the caller has its index)."""
+    if dev is None:
+        dev = _torch.cuda.current_device()
     cache = _cache(space)
     key = ("space", dev)
     if key not in cache:
@@ -245,9 +255,10 @@ def singular_rule_arrays(grid, order, test_support, trial_support):
     return cache[key]
 
 
-def device_singular_rule(grid, order, test_support, trial_support):
-    """Singular pairs of ``grid`` at ``order`` for the given supports, on the device."""
-    dev = _torch.cuda.current_device()
+def device_singular_rule(grid, order, test_support, trial_support, dev=None):
+    """Singular pairs of ``grid`` at ``order`` for the given supports, on the current device (``dev``, as above)."""
+    if dev is None:
+        dev = _torch.cuda.current_device()
     cache = _cache(grid)
     key = ("singular", dev, int(order), _np.asarray(test_support).tobytes(), _np.asarray(trial_support).tobytes())
     if key not in cache:
