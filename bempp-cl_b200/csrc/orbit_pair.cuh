@@ -65,6 +65,8 @@ __device__ __forceinline__ void orbit_offsets(const Geom &g, double e[3][3]) {
     }
 }
 
+// Pairs with r_c < ORBIT_NEAR (R_t + R_s) difference their coordinates (each element's own R: with the grid's largest, or
+// at 1.5, enough ordinary pairs took the branch to cost 4 % in divergence).
 constexpr double ORBIT_NEAR = 1.0;
 
 // A test element in shared memory.

@@ -12,7 +12,8 @@
 //                                                          element; D + g_o e_j squared when r_c < near)
 //   exp(ik r) = exp(ik r_c) exp(ik (r - r_c)), |r - r_c| <= rho R: the second factor by the polynomials of
 // the offset class without range reduction, the first once per element (complex k: the same for the
-// amplitude; class 0 factors nothing and reduces every argument).  `near` = 2.5 R: beyond it r >= 1.7 R and the expanded square loses nothing (r_c^2 / r^2 < 2.1).
+// amplitude; class 0 factors nothing and reduces every argument).  `near` = 2.5 R: beyond it r >= 1.7 R and the
+// expanded square loses nothing (r_c^2 / r^2 < 2.1).
 // Far fields: the phase -k x.y = -k x.c - k g_o x.e_j, the same split.
 //
 // Maxwell: an RWG function's values on one element are alpha y + beta with complex alpha = sum_i x_i l_i and
@@ -25,7 +26,9 @@
 //   magnetic potential   (x - c) x (alpha e_j sigma_j + gamma h0) - (e_j x gamma) sigma_j
 //   far fields           V = gamma g0 + alpha e_j tau_j, W = 2 alpha g0: ik V - x W, ik x x V.
 // The kernels they replace evaluated every source's vector terms and a range-reduced sine / cosine pair.
-// All of them are bound by the FP64 pipe.
+// All of them are bound by the FP64 pipe.  Before -> here: Helmholtz single layer on P1, 8192 elements, 10000 points 1393 ->
+// 1321 us; electric potential, 4232 elements, 4999 points 1898 -> 541 us; electric far field, 8192 elements, 3600
+// directions 1383 -> 529 us.
 #pragma once
 
 #include "potential.cuh"

@@ -9,7 +9,9 @@ namespace bc {
 
 // Row blocks of the P1 and Maxwell sweeps: 32 test elements per CTA, halved while that would leave the GPU
 // under four waves of working CTAs (a symmetric sweep's CTAs below the diagonal exit at once; 3 CTAs per SM), down to
-// one.  The kernels take their chunk height as ceil(ntest / gridDim.y).
+// one.  The kernels take their chunk height as ceil(ntest / gridDim.y).  32 rows against the halved ones: single layer
+// P1, 1152 elements 0.239 and 0.143 ms; electric field, 288 elements 0.094 and 0.075 ms; from 4096 elements on (P1, symmetric) the
+// launch has its four waves and keeps 32, one staging per 32 rows.
 inline unsigned lin_row_blocks(int64_t ntrial, int64_t ntest, bool sym) {
     const int64_t cols = (ntrial + DP0_THREADS - 1) / DP0_THREADS;
     const int64_t wave = (int64_t)bc_sm_count() * 3;
