@@ -24,8 +24,8 @@
 // pairs to fill the GPU.  The flat tables cost a warp 40 bytes per point and lane from L2 (a coincident pair reads
 // 61 KB), which bounded those kernels together with the FP64 work this form divides by four.
 // Bound by the FP64 pipe (the sine / cosine pair of each point).  Flat tables -> this form: P1 hypersingular, 8192
-// elements 0.73 -> 0.38 ms; combined field on DP0, 16200 elements 0.63 -> 0.26 ms; electric field, 2048 elements 0.145 ->
-// 0.075 ms; 24 problems of one batch 1.18 -> 0.65 ms; Laplace on 128 elements 36 -> 9 us.
+// elements 0.63 -> 0.26 ms; combined field on DP0, 16200 elements 0.73 -> 0.38 ms; double layer on P1, 10952 elements
+// 0.89 -> 0.41 ms; electric field, 2048 elements 0.145 -> 0.075 ms; 24 problems of one batch 1.18 -> 0.65 ms; Laplace on 128 elements 36 -> 9 us.
 #pragma once
 
 #include "orbit_pair.cuh"
