@@ -5,11 +5,14 @@
 
 namespace bc {
 
-// Grid (point blocks, element chunks).  The chunk count c minimises the waves times the work of a block,
-//   ceil(pblocks c / slots) (ceil(chunk / 4) + 4)
-// in elements per warp (a block's four warps share its chunk; four elements stand for its start and its
-// final sum), slots = SMs x resident blocks: the grid ends on a full wave.  The fewest elements of a chunk
-// are 8, two per warp.
+// Grid (point blocks, element chunks).  The chunk count c minimises the work over the slots plus one block's,
+//   (pblocks c / slots + 1) (ceil(chunk / 4) + 2)
+// in elements per warp (a block's four warps share its chunk; two elements stand for its start and its
+// final sum), slots = SMs x resident blocks: blocks start as others end, so the last one's length is what is lost.  With
+// whole waves, ceil(pblocks c / slots) (ceil(chunk / 4) + 4), one wave was taken wherever it nearly fitted, and SMs
+// with one block fewer idled: 8192 elements, Helmholtz single layer, 3000 points 0.448 -> 0.392 ms, 10000 points 1.321 ->
+// 1.231 ms, double layer 1.466 -> 1.439 ms, Laplace 3000 points 0.181 -> 0.163 ms, Maxwell electric far field 7000
+// directions 1.018 -> 0.932 ms.  The fewest elements of a chunk are 8, two per warp.
 static cudaError_t orbit_grid(const PotParams &prm, const void *fn, int points, dim3 *grid, int64_t *chunk_elems) {
     int resident = 0;
     const cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, fn, PO_THREADS, 0);
@@ -21,7 +24,7 @@ static cudaError_t orbit_grid(const PotParams &prm, const void *fn, int points, 
     int64_t best = 0, chunk = prm.nsupport;
     for (int64_t c = 1; c <= cmax; ++c) {
         const int64_t elems = (prm.nsupport + c - 1) / c;
-        const int64_t t = ((pblocks * c + slots - 1) / slots) * ((elems + 3) / 4 + 4);
+        const int64_t t = (pblocks * c + slots) * ((elems + 3) / 4 + 2);
         if (c == 1 || t < best) {
             best = t;
             chunk = elems;
