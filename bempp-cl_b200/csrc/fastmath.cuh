@@ -105,6 +105,9 @@ __device__ __forceinline__ double rsqrt64(double x) {
     return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
+// A distance from its square; 0 below 1e-150, where rsqrt64 is NaN (0, subnormal numbers) or soon will be.
+__device__ __forceinline__ double dist64(double r2) { return r2 > 1e-300 ? r2 * rsqrt64(r2) : 0.0; }
+
 // |x| <= 1 without reduction (callers know the bound).
 __device__ __forceinline__ void sincos_small64(double x, double *s, double *c) {
     constexpr double ps[] = BC_SIN_SMALL64;

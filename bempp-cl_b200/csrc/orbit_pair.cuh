@@ -161,7 +161,7 @@ __device__ __forceinline__ void orbit_pair(const OrbitTest &t, const TRIAL &s, c
     p.far = p.rc2 >= near * near;
     p.krc = p.kirc = 0.0;
     if (CLS > 0 && FAM != FAM_LAPLACE) {
-        const double rc = p.rc2 * rsqrt64(p.rc2);
+        const double rc = dist64(p.rc2);  // elements of two grids may share a centroid
         p.krc = kr * rc;
         if (CK) p.kirc = ki * rc;
     }

@@ -201,8 +201,7 @@ __global__ void __launch_bounds__(PO_THREADS) potential_orbit(PotParams prm, Orb
 #pragma unroll
                     for (int d = 0; d < 3; ++d) D[j][d] = c[d] - x[j][d];
                     const double rc2 = fma(D[j][2], D[j][2], fma(D[j][1], D[j][1], D[j][0] * D[j][0]));
-                    rc_[j] = rc2 > 0.0 ? rc2 * rsqrt64(rc2) : 0.0;  // a point may sit on a centroid
-                    if (CLS == 0) rc_[j] = 0.0;
+                    rc_[j] = CLS > 0 ? dist64(rc2) : 0.0;  // a point may sit on a centroid
                     ph[j] = HELM || MH ? k * rc_[j] : 0.0;
                     if (rc2 >= near2) {
                         const double a0 = fma(D[j][2], e0[2], fma(D[j][1], e0[1], D[j][0] * e0[0]));

@@ -112,3 +112,64 @@ def test_rule_in_another_order(case, interface, monkeypatch):
     monkeypatch.setattr(assembly, "regular_rule", lambda o: rule)
     got = _operator(*case, grid, 1.2, device_interface=interface)[0].weak_form().A
     assert rel_fro(got, ref) < 1e-12
+
+
+def _octahedron():
+    """Eight triangles with vertices at +-1 on the axes (dyadic coordinates)."""
+    from bempp_cuda.grid import Grid
+    from bempp_cuda.shapes import sphere_arrays
+
+    vertices, elements = sphere_arrays(0)
+    return Grid(np.round(vertices), elements)
+
+
+def _midpoint_refined(grid):
+    """Every triangle in four by its edge midpoints, left in its plane: the central one has its parent's centroid."""
+    from bempp_cuda.grid import Grid
+
+    v, e = np.asarray(grid.vertices), np.asarray(grid.elements)
+    a, b, c = (v[:, e[i]] for i in range(3))
+    ab, bc, ca = 0.5 * (a + b), 0.5 * (b + c), 0.5 * (c + a)
+    corners = np.concatenate([np.stack(t) for t in ((a, ab, ca), (ab, b, bc), (ca, bc, c), (ab, bc, ca))], axis=2)
+    points, index = np.unique(corners.transpose(0, 2, 1).reshape(-1, 3), axis=0, return_inverse=True)
+    return Grid(np.ascontiguousarray(points.T), np.ascontiguousarray(index.reshape(3, -1)))
+
+
+COMMON = [c for c in OPERATORS if c[2] in ("P", "RWG") and c[0] != "laplace"] + [
+    ("modified_helmholtz", "single_layer", "P", 1), ("modified_helmholtz", "double_layer", "P", 1)]
+
+
+def _united(a, b):
+    """Both triangulations in one grid (the oracle takes one), no vertex shared."""
+    from bempp_cuda.grid import Grid
+
+    return Grid(np.concatenate([a.vertices, b.vertices], axis=1),
+                np.concatenate([a.elements, b.elements + a.vertices.shape[1]], axis=1))
+
+
+@pytest.mark.parametrize("case", COMMON)
+def test_common_centroids(oracle, case):
+    """Trial and test elements of two grids with the same centroid: r_c = 0, and no two of their points meet."""
+    from bempp_cuda import operators
+    from bempp_cuda.device import device_grid
+    from bempp_cuda.space import function_space
+    from cases import oracle_dense
+
+    equation, name, kind, degree = case
+    coarse = _octahedron()
+    fine = _midpoint_refined(coarse)
+    both, nc = _united(coarse, fine), coarse.number_of_elements
+    test_kind = "SNC" if kind == "RWG" else kind
+    domain, dual = function_space(coarse, kind, degree), function_space(fine, test_kind, degree)
+    domain1 = function_space(both, kind, degree, support_elements=np.arange(nc))
+    dual1 = function_space(both, test_kind, degree, support_elements=np.arange(nc, both.number_of_elements))
+    bound = device_grid(coarse).radius + device_grid(fine).radius
+    factory = getattr(getattr(operators.boundary, equation), name)
+    for theta in (0.4, 0.9, 2.5):  # offset classes 2, 1, 0
+        for k in (theta / bound,) if equation == "modified_helmholtz" else (theta / bound, (1.0 + 0.8j) * theta / bound):
+            got = factory(domain, domain, dual, k).weak_form().A
+            op = factory(domain1, domain1, dual1, k)
+            ref = oracle_dense(oracle, op, domain1, dual1)
+            assert np.isfinite(ref).all() and np.isfinite(got).all()
+            assert rel_fro(got, ref) < 1e-12
+            assert rel_fro(op.weak_form().A, ref) < 1e-12

@@ -111,3 +111,19 @@ def test_rule_in_another_order(oracle, path, monkeypatch):
     rule = (np.ascontiguousarray(pts[order]), np.ascontiguousarray(wts[order]))
     monkeypatch.setattr(assembly, "regular_rule", lambda o: rule)
     assert rel_fro(op.evaluate_device(c).cpu().numpy(), got) < 1e-12
+
+
+@pytest.mark.parametrize("path", [p for p in OPERATORS if p.startswith("potential") and "laplace" not in p])
+def test_at_a_centroid(oracle, path):
+    """Points on a centroid and so close to one that the squared distance is a subnormal number."""
+    from bempp_cuda.grid import Grid
+    from bempp_cuda.shapes import sphere_arrays
+    from bempp_cuda.space import function_space
+
+    vertices, elements = sphere_arrays(0)
+    vertices = 3.0 * np.round(vertices) - 1.0  # the face at (3, 0, 0), (0, 3, 0), (0, 0, 3) moves to the centroid 0
+    space = function_space(Grid(vertices, elements), *(("RWG", 0) if "maxwell" in path else ("P", 1)))
+    points = np.array([[0.0, 1e-160, 1e-160], [0.0, 0.0, -1e-161], [0.0, 0.0, 0.0]])
+    for k in (0.1,) if "modified" in path else (0.1, 0.1 + 0.06j):
+        got, _, _ = _run(path, space, points, k, oracle, 1e-12)
+        assert np.isfinite(got).all()
