@@ -155,6 +155,7 @@ __device__ __forceinline__ void load_trial_sym64(const RegParams &prm, const Qua
     tr.sv2 = __ldg(prm.sel + 3 * s + 2);
     if (form_orbit(FORM)) {
         tr.o = park_orbit_trial<DP0_THREADS>(prm.sg, prm.sne, s, tr.gs, park);
+        orbit_fence();
     } else {
 #pragma unroll
         for (int q = 0; q < NQ6; ++q) to_global(tr.gs, rule.x[q], rule.y[q], tr.y[q]);

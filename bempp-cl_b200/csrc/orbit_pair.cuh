@@ -95,9 +95,14 @@ __device__ __forceinline__ void stage_orbit(const double *__restrict__ geom, int
     o.radius = ORBIT_NEAR * sqrt(r2);
 }
 
+// OrbitTrial::ld is inline assembly that names no memory (a "memory" clobber on every load would hold back the
+// scheduling of the sums), so the order of a thread's stores to its column and its loads is stated here: the fence comes
+// between the loads of one element and the stores of the next, and between the last store and the first load.
+__device__ __forceinline__ void orbit_fence() { asm volatile("" ::: "memory"); }
+
 // A thread's trial element, parked in shared memory (field-major, one column per thread): the sums over the point
 // pairs want the registers, and a field is read at most once per test vertex.  Loads are volatile so that they
-// stay inside the loop over the test elements.
+// stay inside the loop over the test elements (orbit_fence before the first).
 constexpr int OT_C = 0, OT_F = 3, OT_FF = 9, OT_N = 12, OT_IE = 15, OT_RAD = 16, OT_FIELDS = 17;
 
 template <int THREADS>
@@ -128,6 +133,7 @@ struct OrbitTrial {
 template <int THREADS>
 __device__ __forceinline__ OrbitTrial<THREADS> park_orbit_trial(const double *__restrict__ geom, int64_t ne, int64_t s,
                                                                 const Geom &g, double *park) {
+    orbit_fence();
     double f[3][3];
     orbit_offsets(g, f);
     double *o = park + threadIdx.x;

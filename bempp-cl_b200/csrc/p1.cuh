@@ -121,6 +121,7 @@ __global__ void __launch_bounds__(DP0_THREADS, (p1_min_blocks<K, SYM>())) regula
         park[MULT + j][threadIdx.x] = prm.smult[s * NS + j];
         park[COL + j][threadIdx.x] = __longlong_as_double((int64_t)prm.sl2g[s * NS + j]);
     }
+    orbit_fence();
     const double kr = prm.p[0], ki = CK ? prm.p[1] : 0.0;
 
 #pragma unroll 1

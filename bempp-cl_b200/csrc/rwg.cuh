@@ -435,6 +435,7 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_rwg_orbit(RegParams prm, 
         park[FAC + j][threadIdx.x] = prm.smult[s * 3 + j] * edge_length(prm.sg, prm.sne, s, j);
         park[COL + j][threadIdx.x] = __longlong_as_double((int64_t)prm.sl2g[s * 3 + j]);
     }
+    orbit_fence();
     const double kr = prm.p[0], ki = prm.p[1];
 
 #pragma unroll 1
