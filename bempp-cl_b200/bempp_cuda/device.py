@@ -95,8 +95,27 @@ def host_space_arrays(space):
     }
 
 
-class DeviceGrid(object):
+class _PointsAtTensors(object):
+    """Device copies that keep argument records or raw pointers into their own tensors: a copied or unpickled object
+    gets its own, pointing at its own tensors."""
+
+    _POINTERS = ()  # the attributes that _point_at_tensors sets
+
+    def _point_at_tensors(self):
+        raise NotImplementedError
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k not in self._POINTERS}
+
+    def __setstate__(self, state):
+        self.__dict__.update(state)
+        self._point_at_tensors()
+
+
+class DeviceGrid(_PointsAtTensors):
     """Vertices, elements and the per-element geometry record on the device."""
+
+    _POINTERS = ("_record",)
 
     def __init__(self, grid):
         vertices, elements = host_grid_arrays(grid)
@@ -120,6 +139,9 @@ class DeviceGrid(object):
         corners = vertices[elements]  # (ne, 3, 3)
         centroids = corners.mean(axis=1, keepdims=True)
         self.radius = float(_np.sqrt(((corners - centroids) ** 2).sum(axis=2)).max()) if self.nelements else 0.0
+        self._point_at_tensors()
+
+    def _point_at_tensors(self):
         self._record = _lib.GridRec(self.nvertices, self.nelements, ptr(self.geom), ptr(self.elements))
 
     def record(self):
@@ -138,8 +160,10 @@ def _shared_on_grid(grid, name, array, dtype):
     return cache[key]
 
 
-class DeviceSpace(object):
+class DeviceSpace(_PointsAtTensors):
     """Support list and dof maps of one space on the device."""
+
+    _POINTERS = ("_record",)
 
     def __init__(self, space):
         h = host_space_arrays(space)
@@ -154,6 +178,9 @@ class DeviceSpace(object):
         self.mult = _shared_on_grid(grid, "mult", h["mult"], _torch.float64)
         self.normal_mult = _shared_on_grid(grid, "normal_mult", h["normal_mult"], _torch.int32)
         self.h2d_bytes = sum(h[name].nbytes for name in ("support", "l2g", "mult", "normal_mult"))
+        self._point_at_tensors()
+
+    def _point_at_tensors(self):
         self._record = _lib.Space(
             self.shapeset,
             self.nshape,
@@ -171,8 +198,10 @@ class DeviceSpace(object):
         return self._record
 
 
-class DeviceSingularRule(object):
+class DeviceSingularRule(_PointsAtTensors):
     """Flattened Sauter-Schwab pair list and point tables on the device."""
+
+    _POINTERS = ("_tables", "_pairs")
 
     def __init__(self, arrays):
         tp, sp, w, te, se, toff, soff, woff, npts = arrays
@@ -190,6 +219,9 @@ class DeviceSingularRule(object):
         self.h2d_bytes = tp.nbytes + sp.nbytes + 8 * len(w) + sum(a.nbytes for a in ints)
         self._host_ints = ints
         self._by_test = None
+        self._point_at_tensors()
+
+    def _point_at_tensors(self):
         self._tables = tuple(t.data_ptr() for t in (self.test_points, self.trial_points, self.weights))
         self._pairs = tuple(t.data_ptr() for t in (self.test_elements, self.trial_elements, self.test_offsets,
                                                    self.trial_offsets, self.weights_offsets, self.npoints))
