@@ -59,8 +59,8 @@ inline int sym_form(int kernel, const double *params, double radius_sum, bool or
     const double kmax = ck ? fmax(fabs(params[0]), fabs(params[1])) : fabs(params[0]);
     const int cls = offset_class64(kmax * radius_sum * (orbits ? orbit.rho : 1.0));
     if (!ck && !modhelm) return SYM_POINTS + cls;
-    // (the orbit form divides by Re k)
-    if (!orbits || params[0] == 0.0) return ck ? SYM_POINTS_CK : SYM_POINTS;
+    // (the orbit form sums h / Re k: finite above this bound for |k| and 1 / r up to 1e60)
+    if (!orbits || fabs(params[0]) < 1e-100) return ck ? SYM_POINTS_CK : SYM_POINTS;
     return (ck ? SYM_ORBIT_CK : SYM_ORBIT) + cls;
 }
 

@@ -173,3 +173,12 @@ def test_common_centroids(oracle, case):
             assert np.isfinite(ref).all() and np.isfinite(got).all()
             assert rel_fro(got, ref) < 1e-12
             assert rel_fro(op.weak_form().A, ref) < 1e-12
+
+
+@pytest.mark.parametrize("name", ["double_layer", "adjoint_double_layer"])
+@pytest.mark.parametrize("k", [1e-310 + 0.9j, 1e-30 + 0.9j])
+def test_nearly_imaginary_wavenumber(oracle, name, k):
+    """A real part too small to divide by."""
+    from bempp_cuda.shapes import ellipsoid
+
+    _check(oracle, ("helmholtz", name, "DP", 0), ellipsoid(2, 1.0, 0.8, 1.2), k, 1e-12)
