@@ -1,35 +1,19 @@
 // Launches of the FP64 potential and far-field kernels with the two-orbit rule (potential_orbit.cuh).
 #include <algorithm>
 
+#include "potential_chunk.h"
 #include "potential_orbit.cuh"
 
 namespace bc {
 
-// Grid (point blocks, element chunks).  The chunk count c minimises the work over the slots plus one block's,
-//   (pblocks c / slots + 1) (ceil(chunk / 4) + 2)
-// in elements per warp (a block's four warps share its chunk; two elements stand for its start and its
-// final sum), slots = SMs x resident blocks: blocks start as others end, so the last one's length is what is lost.  With
-// whole waves, ceil(pblocks c / slots) (ceil(chunk / 4) + 4), one wave was taken wherever it nearly fitted, and SMs
-// with one block fewer idled: 8192 elements, Helmholtz single layer, 3000 points 0.448 -> 0.392 ms, 10000 points 1.321 ->
-// 1.231 ms, double layer 1.466 -> 1.439 ms, Laplace 3000 points 0.181 -> 0.163 ms, Maxwell electric far field 7000
-// directions 1.018 -> 0.932 ms.  The fewest elements of a chunk are 8, two per warp.
+// Grid (point blocks, element chunks).
 static cudaError_t orbit_grid(const PotParams &prm, const void *fn, int points, dim3 *grid, int64_t *chunk_elems) {
     int resident = 0;
     const cudaError_t err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, fn, PO_THREADS, 0);
     if (err != cudaSuccess) return err;
     const int64_t slots = (int64_t)bc_sm_count() * std::max(resident, 1);
     const int64_t pblocks = (prm.npoints + points - 1) / points;
-    int64_t cmax = std::min<int64_t>((prm.nsupport + 7) / 8, 65535);
-    cmax = std::max<int64_t>(1, std::min<int64_t>(cmax, 8 * ((slots + pblocks - 1) / pblocks)));
-    int64_t best = 0, chunk = prm.nsupport;
-    for (int64_t c = 1; c <= cmax; ++c) {
-        const int64_t elems = (prm.nsupport + c - 1) / c;
-        const int64_t t = (pblocks * c + slots) * ((elems + 3) / 4 + 2);
-        if (c == 1 || t < best) {
-            best = t;
-            chunk = elems;
-        }
-    }
+    const int64_t chunk = potential_chunk(prm.nsupport, pblocks, slots);
     *chunk_elems = chunk;
     *grid = dim3((unsigned)pblocks, (unsigned)((prm.nsupport + chunk - 1) / chunk));
     return cudaSuccess;
