@@ -55,11 +55,11 @@ bool potential_orbit_has(int assembly, int kernel) {
 cudaError_t launch_potential_orbit(const PotParams &prm, const OrbitRule &rule, int assembly, int kernel,
                                    double phase_radius, cudaStream_t st) {
     const bool maxwell = assembly != BEMPPCUDA_ASM_SCALAR;
-    const unsigned blocks = (unsigned)((prm.nsupport + PO_THREADS - 1) / PO_THREADS);
+    const unsigned blocks = (unsigned)((prm.nsupport + PO_ELEMS - 1) / PO_ELEMS);
     if (maxwell)
-        potential_elements<true><<<blocks, PO_THREADS, 0, st>>>(prm, rule);
+        potential_elements<true><<<blocks, PO_ELEMS, 0, st>>>(prm, rule);
     else
-        potential_elements<false><<<blocks, PO_THREADS, 0, st>>>(prm, rule);
+        potential_elements<false><<<blocks, PO_ELEMS, 0, st>>>(prm, rule);
     const cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     const bool far = kernel == BEMPPCUDA_FARFIELD_SLP || kernel == BEMPPCUDA_FARFIELD_DLP;
