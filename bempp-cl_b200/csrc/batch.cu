@@ -151,7 +151,8 @@ template <int K>
 __global__ void __launch_bounds__(DP0_THREADS) regular_batch(const BatchDev *__restrict__ probs, int nprob,
                                                               int64_t total_tiles,
                                                               unsigned long long *__restrict__ counter,
-                                                              QuadRule rule, OrbitConsts oc, int orbits) {
+                                                              const __grid_constant__ QuadRule rule, OrbitConsts oc,
+                                                              int orbits) {
     __shared__ TileShared sh;
     __shared__ long long s_tile;
     while (true) {

@@ -503,6 +503,24 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
+// Two-orbit sweeps, pairs whose points may meet (r_c < MIXED_NEAR (R_t + R_s); the points lie within 0.725 R of their
+// centroid).  There the expanded square r_c^2 + s loses (r_c / r)^2 of FP32's digits, so the coordinates are
+// differenced: -r'^2 of the test point at x = D - g_p e_i and the two trial points (one per orbit) of vertex j.  No pair
+// of a quasi-uniform mesh is that near without sharing a vertex.  Errors relative to FP64, expanded square ->
+// differenced, ellipsoids of 512 elements: axes 1, 1, 0.01, k = 1.3, double layer on P1 1.2e-5 -> 5.4e-8, magnetic field
+// 2.4e-5 -> 1.1e-7; axes 1, 0.03, 0.03, single layer on DP0 2.2e-7 -> 6.6e-8.
+constexpr double MIXED_NEAR = 0.8;
+__device__ __forceinline__ float2 near_mr2(const float x[3], const float f[2][3], int j, float2 g2) {
+    float2 r2 = b2(0.f);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const float fj = j == 0 ? f[0][d] : j == 1 ? f[1][d] : -(f[0][d] + f[1][d]);
+        const float2 v = fma2(b2(fj), g2, b2(x[d]));
+        r2 = d == 0 ? mul2(v, v) : fma2(v, v, r2);
+    }
+    return f2(-r2.x, -r2.y);
+}
+
 template <int PHC>
 __device__ __forceinline__ void sincos2(float2 x, float2 *s, float2 *c) {
     if (PHC == 2) {

@@ -411,9 +411,10 @@ struct TestBlock32q {
     float e[DP0_TCHUNK][3][3];
     float hge[DP0_TCHUNK][2][3];
     double c[DP0_TCHUNK][3];
-    float4 n[DP0_TCHUNK];  // unit normal (fourth entry unused)
+    float4 n[DP0_TCHUNK];  // unit normal, MIXED_NEAR R
     double ie[DP0_TCHUNK];
     int v[DP0_TCHUNK][3];
+    float srad[DP0_THREADS];  // MIXED_NEAR R of each thread's trial element
 };
 
 // sin / cos of the point-pair phase offsets of the symmetric sweep (|x| <= 1/2 for phase class
@@ -446,6 +447,260 @@ __device__ __forceinline__ void sincos2_sym(float2 x, float2 *s, float2 *c) {
     }
 }
 
+// One thread's trial element, lengths in units of 1/kappa.
+struct MixedTrial {
+    float f[2][3];  // vertex offsets f_0, f_1 (f_2 = -f_0 - f_1)
+    float2 hgf[3];  // -g_q^2 |f_j|^2 / 2 of both orbits
+    float n[3], rad;  // normal, MIXED_NEAR R
+    double c[3], ie;
+    int v[3];
+};
+
+template <int K>
+__device__ __forceinline__ double mixed_kappa(const RegParams &prm) {
+    // units of 1/kappa: Re k (Helmholtz), omega (modified Helmholtz), 1 (Laplace); callers guarantee kappa > 0
+    return SymTraits<K>::helm || SymTraits<K>::modhelm ? prm.p[0] : 1.0;
+}
+// The orbits' offset factors: the first point of an orbit belongs to vertex 2.
+__device__ __forceinline__ double mixed_g(const QuadRule &rule, int o) { return 1.0 - 3.0 * rule.x[o * (NQ6 / 2)]; }
+
+template <int K>
+__device__ __forceinline__ void load_trial_mixed(const RegParams &prm, const QuadRule &rule, int64_t si, MixedTrial &tr) {
+    const double kap = mixed_kappa<K>(prm), g0d = mixed_g(rule, 0), g1d = mixed_g(rule, 1);
+    const int64_t s = prm.ssup[si];
+    Geom gs;
+    load_geom(prm.sg, prm.sne, s, prm.snm ? (double)prm.snm[s] : 1.0, gs);
+    double fd[3][3], m2 = 0.0;
+    orbit_offsets(gs, fd);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const double ff = odot(fd[j], fd[j]), m = -0.5 * kap * kap * ff;
+        m2 = fmax(m2, ff);
+        tr.hgf[j] = f2((float)(g0d * g0d * m), (float)(g1d * g1d * m));
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        tr.f[0][d] = (float)(kap * fd[0][d]);
+        tr.f[1][d] = (float)(kap * fd[1][d]);
+        tr.n[d] = (float)gs.n[d];
+        tr.c[d] = __ldg(prm.sg + (22 + d) * prm.sne + s);
+        tr.v[d] = __ldg(prm.sel + 3 * s + d);
+    }
+    tr.rad = (float)(MIXED_NEAR * kap * sqrt(m2));
+    tr.ie = gs.ie;
+}
+
+// The entries A_ij and A_ji of the test element tt of the block and the trial element, D = kappa (c_s - c_t).  NEAR:
+// differenced coordinates and no Newton step: theta = r' - r_c' is as good as r' there.
+template <int K, int PHC, bool CK, bool NEAR>
+__device__ __forceinline__ void mixed_pair(const RegParams &prm, const QuadRule &rule, const TestBlock32q &sb, int tt,
+                                           const MixedTrial &tr, double D0, double D1, double D2, double rc2,
+                                           double &a_re, double &a_im, double &b_re, double &b_im) {
+    using ST = SymTraits<K>;
+    const double kap = mixed_kappa<K>(prm);
+    const double betd = CK ? prm.p[1] / prm.p[0] : 0.0;
+    const float2 bet2 = b2((float)betd);
+    const float go[2] = {(float)mixed_g(rule, 0), (float)mixed_g(rule, 1)};
+    const float2 g2 = f2(go[0], go[1]);
+    const float(&f)[2][3] = tr.f;
+    const float2(&hgf)[3] = tr.hgf;
+    const float sn0 = tr.n[0], sn1 = tr.n[1], sn2 = tr.n[2];
+    const double ek_r = (K == BEMPPCUDA_HELMHOLTZ_COMBINED) ? kap * prm.p[2] : kap;
+    const double ek_i = (K == BEMPPCUDA_HELMHOLTZ_COMBINED) ? kap * prm.p[3] : 0.0;
+    const double k2d = kap * kap;
+    // weights: w_b for the second test orbit, w_a / w_b applied in FP32 to the first; the trial orbits' at the end
+    const double wb = rule.w[NQ6 - 1];
+    const float2 rho2 = b2((float)(rule.w[0] / wb));
+    const float wqa = rule.wf[0], wqb = rule.wf[NQ6 - 1];
+    const auto fdot = [](const float a[3], float b0, float b1, float b2_) {
+        return fmaf(a[2], b2_, fmaf(a[1], b1, a[0] * b0));
+    };
+    const double rc = NEAR ? dist64(rc2) : rc2 * rsqrt64(rc2);
+    float ph_s = 0.f, ph_c = 1.f;
+    if (ST::helm) phase_reduced32(rc, &ph_s, &ph_c);
+    // e^{-beta r_c'} (complex k), e^{-r_c'} (modified Helmholtz)
+    const double amp = CK ? exp_neg_reduced(betd * rc) : (ST::modhelm ? exp_neg_reduced(rc) : 1.0);
+    const float D0f = (float)D0, D1f = (float)D1, D2f = (float)D2, rcf = (float)rc;
+    const float2 rc_2 = b2(rcf), mrc_2 = b2(-rcf), mrc2_2 = b2(-(float)rc2);
+    // k (y - x).n_s = Dn - g_p e_i . n_s, one factor per test point; k (x - y).n_t = -Dt - g_q f_j . n_t,
+    // one per trial point
+    float Dn = 0.f;
+    float2 ynt[3];
+    if (ST::dlp_part) {
+        const float4 tn = sb.n[tt];
+        const float mDt = -fmaf(D2f, tn.z, fmaf(D1f, tn.y, D0f * tn.x));
+        const float m0 = -fdot(f[0], tn.x, tn.y, tn.z), m1 = -fdot(f[1], tn.x, tn.y, tn.z);
+        ynt[0] = fma2(b2(m0), g2, b2(mDt));
+        ynt[1] = fma2(b2(m1), g2, b2(mDt));
+        ynt[2] = fma2(b2(-(m0 + m1)), g2, b2(mDt));
+        Dn = fmaf(D2f, sn2, fmaf(D1f, sn1, D0f * sn0));
+    }
+    float2 hA[3];  // -A_q / 2
+    if (!NEAR) {
+        const float a0 = -fdot(f[0], D0f, D1f, D2f), a1 = -fdot(f[1], D0f, D1f, D2f);
+        hA[0] = fma2(b2(a0), g2, hgf[0]);
+        hA[1] = fma2(b2(a1), g2, hgf[1]);
+        hA[2] = fma2(b2(-(a0 + a1)), g2, hgf[2]);
+    }
+    float E[3][3], De[3], en[3];  // e_i . f_j, D . e_i, e_i . n_s
+    if (!NEAR) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float e0 = sb.e[tt][i][0], e1 = sb.e[tt][i][1], e2 = sb.e[tt][i][2];
+            De[i] = fmaf(D2f, e2, fmaf(D1f, e1, D0f * e0));
+            if (ST::dlp_part) en[i] = fmaf(sn2, e2, fmaf(sn1, e1, sn0 * e0));
+            E[i][0] = fdot(f[0], e0, e1, e2);
+            E[i][1] = fdot(f[1], e0, e1, e2);
+            E[i][2] = -(E[i][0] + E[i][1]);
+        }
+        De[2] = -(De[0] + De[1]);
+        if (ST::dlp_part) en[2] = -(en[0] + en[1]);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) E[2][j] = -(E[0][j] + E[1][j]);
+    }
+    float2 s0r = b2(0.f), s0m = b2(0.f), um = b2(0.f), ui = b2(0.f), vm = b2(0.f), vi = b2(0.f);
+#pragma unroll (NEAR ? 1 : NQ6)
+    for (int p = 0; p < NQ6; ++p) {
+        const int i = p % 3, op = p / 3;
+        if (p == NQ6 / 2) {  // second orbit: the first orbit's sums times w_a / w_b
+            s0r = mul2(s0r, rho2);
+            s0m = mul2(s0m, rho2);
+            um = mul2(um, rho2);
+            ui = mul2(ui, rho2);
+            vm = mul2(vm, rho2);
+            vi = mul2(vi, rho2);
+        }
+        const float gp = op == 0 ? go[0] : go[1];
+        float x[3];  // NEAR: D - g_p e_i
+        float2 hB, gp2, cp2 = b2(0.f);
+        if (NEAR) {
+            x[0] = fmaf(-gp, sb.e[tt][i][0], D0f);
+            x[1] = fmaf(-gp, sb.e[tt][i][1], D1f);
+            x[2] = fmaf(-gp, sb.e[tt][i][2], D2f);
+            if (ST::dlp_part) cp2 = b2(fdot(x, sn0, sn1, sn2));
+        } else {
+            hB = b2(fmaf(gp, De[i], sb.hge[tt][op][i]));  // -B_p / 2
+            gp2 = f2(gp * go[0], gp * go[1]);
+            if (ST::dlp_part) cp2 = b2(fmaf(-gp, en[i], Dn));
+        }
+        float2 pum = b2(0.f), pui = b2(0.f);  // sums over q of the A_ij double-layer factors, times cp per p
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            float2 hs, mr2;  // -s / 2, -r'^2
+            if (NEAR) {
+                mr2 = near_mr2(x, f, j, g2);
+            } else {
+                hs = fma2(b2(E[i][j]), gp2, add2(hA[j], hB));
+                mr2 = fma2(hs, b2(2.f), mrc2_2);
+            }
+            const float2 rinv = f2(rsqrt_approx(-mr2.x), rsqrt_approx(-mr2.y));
+            // -theta
+            float2 mt = b2(0.f);
+            if (ST::helm || ST::modhelm) {
+                mt = fma2(mr2, rinv, rc_2);
+                if (!NEAR) mt = fma2(fma2(mt, fma2(mt, b2(0.5f), mrc_2), hs), rinv, mt);
+            }
+            if (!ST::helm) {
+                // modified Helmholtz: e^{-theta} per pair (e^{-r_c'} per element pair), the double
+                // layers' (1 + r') e^{-theta}
+                float2 am = b2(1.f), am1 = b2(1.f);
+                if (ST::modhelm) {
+                    am = f2(__expf(mt.x), __expf(mt.y));
+                    am1 = mul2(am, add2(b2(1.f), mul2(mul2(mr2, rinv), b2(-1.f))));
+                }
+                if (ST::slp_part) s0r = ST::modhelm ? fma2(rinv, am, s0r) : add2(rinv, s0r);
+                if (ST::dlp_part) {
+                    float2 fr = mul2(mul2(rinv, rinv), rinv);
+                    if (ST::modhelm) fr = mul2(fr, am1);
+                    pum = add2(fr, pum);
+                    vm = fma2(fr, ynt[j], vm);
+                }
+            } else {
+                float2 ms, cs;  // -sin, cos of theta
+                sincos2_sym<PHC>(mt, &ms, &cs);
+                if (CK) {
+                    const float2 am = f2(__expf(bet2.x * mt.x), __expf(bet2.x * mt.y));
+                    cs = mul2(cs, am);
+                    ms = mul2(ms, am);
+                }
+                if (ST::slp_part) {
+                    s0r = fma2(rinv, cs, s0r);
+                    s0m = fma2(rinv, ms, s0m);
+                }
+                if (ST::dlp_part) {
+                    const float2 fr = mul2(rinv, rinv);
+                    const float2 rb = CK ? add2(rinv, bet2) : rinv;  // 1 / r' (+ beta)
+                    const float2 mh1 = fma2(mul2(rb, b2(-1.f)), cs, ms);  // -h1
+                    const float2 h2 = fma2(rb, ms, cs);
+                    const float2 gt = mul2(fr, ynt[j]);
+                    pum = fma2(fr, mh1, pum);
+                    pui = fma2(fr, h2, pui);
+                    vm = fma2(gt, mh1, vm);
+                    vi = fma2(gt, h2, vi);
+                }
+            }
+        }
+        if (ST::dlp_part) {
+            um = fma2(cp2, pum, um);
+            if (ST::helm) ui = fma2(cp2, pui, ui);
+        }
+    }
+    // entry = w_b [kappa eta S0 + kappa^2 (-h1 sum + i h2 sum)], rotated by exp(i r_c') and scaled; um and vm
+    // hold the -h1 sums (Helmholtz) or the sums of w (d'.n) / r'^3 (real kernels)
+    const auto orbits = [&](float2 v) { return (double)fmaf(wqa, v.x, wqb * v.y); };
+    double sr = 0.0, sim = 0.0;
+    if (ST::slp_part) {
+        const double xr = orbits(s0r), xi = ST::helm ? -orbits(s0m) : 0.0;
+        sr = fma(ek_r, xr, -ek_i * xi);
+        sim = fma(ek_r, xi, ek_i * xr);
+    }
+    double dr = 0.0, di = 0.0, er = 0.0, ei = 0.0;
+    if (ST::dlp_part) {
+        const double sg = ST::helm ? k2d : -k2d;
+        dr = sg * orbits(um);
+        er = sg * orbits(vm);
+        if (ST::helm) {
+            di = k2d * orbits(ui);
+            ei = k2d * orbits(vi);
+        }
+    }
+    if (ST::swap) {
+        a_re = er;
+        a_im = ei;
+        b_re = dr;
+        b_im = di;
+    } else {
+        a_re = sr + dr;
+        a_im = sim + di;
+        b_re = sr + er;
+        b_im = sim + ei;
+    }
+    const double scale = BC_INV_4PI * sb.ie[tt] * tr.ie * wb * amp;
+    const double pc = (double)ph_c, ps = (double)ph_s;
+    double rot = a_re * pc - a_im * ps;
+    a_im = (a_re * ps + a_im * pc) * scale;
+    a_re = rot * scale;
+    rot = b_re * pc - b_im * ps;
+    b_im = (b_re * ps + b_im * pc) * scale;
+    b_re = rot * scale;
+}
+
+// A near pair: a function of its own that loads the trial element again, called after the sweep's own evaluation, so
+// that the sweep keeps its registers and schedule.  On meshes without such pairs it costs the combined field nothing
+// (32768 elements 21.12 -> 21.08 ms), other kernels up to 2 %; branching around the sweep's evaluation 1 - 2 %, inlined or
+// collected for after the sweep 2 - 10 %.
+template <int K, int PHC, bool CK>
+__device__ __noinline__ void mixed_near_pair(const RegParams &prm, const QuadRule &rule, const TestBlock32q &sb, int tt,
+                                             int64_t si, double (&ab)[4]) {
+    const double kap = mixed_kappa<K>(prm);
+    MixedTrial tr;
+    load_trial_mixed<K>(prm, rule, si, tr);
+    const double D0 = kap * (tr.c[0] - sb.c[tt][0]), D1 = kap * (tr.c[1] - sb.c[tt][1]),
+                 D2 = kap * (tr.c[2] - sb.c[tt][2]);
+    mixed_pair<K, PHC, CK, true>(prm, rule, sb, tt, tr, D0, D1, D2, fma(D2, D2, fma(D1, D1, D0 * D0)), ab[0], ab[1],
+                                 ab[2], ab[3]);
+}
+
 // Packed mixed precision in wavenumber-scaled units with the two-orbit rule (orbit.cuh).  The trial points of
 // one vertex, one of each orbit, travel together in f32x2 operations, so an orbit's weight is applied to its
 // half of the sums at the end of the pair, and the offset products need one dot product per pair of vertices:
@@ -462,7 +717,8 @@ __device__ __forceinline__ void sincos2_sym(float2 x, float2 *s, float2 *c) {
 //
 // Per element pair: the centroid offset D and |D|^2 in FP64 (r_c' for the phase), FP32 copies for the
 // point-pair terms; elements whose centroids are farther apart than prm.near_r cannot share a vertex, so the
-// vertex test runs only for near pairs; the pair phase exp(i r_c') by phase_reduced32.  The FP32 sums of the
+// vertex test runs only for closer pairs, and of those the near ones difference the coordinates (near_mr2, dp0.cuh);
+// the pair phase exp(i r_c') by phase_reduced32.  The FP32 sums of the
 // first test orbit are scaled by w_a / w_b when the second begins, and everything is converted to FP64 once,
 // times w_b.
 // Bound by the FMA pipe with the special-function unit close behind.  Combined field, 32768 elements, k = 10: 22.02 ->
@@ -474,241 +730,63 @@ __device__ __forceinline__ void sincos2_sym(float2 x, float2 *s, float2 *c) {
 template <int K, int PHC, bool STRIPE = false, bool CK = false>
 __device__ __forceinline__ void regular_dp0_mixed_sym_tile(const RegParams &prm, const QuadRule &rule,
                                                          int64_t tile_x, int64_t t0, int rows, TestBlock32q &sb) {
-    using ST = SymTraits<K>;
-    static_assert(!CK || ST::helm, "complex wavenumber: the Helmholtz kernels");
-    // units of 1/kappa: Re k (Helmholtz), omega (modified Helmholtz), 1 (Laplace); callers guarantee kappa > 0
-    const double kap = ST::helm || ST::modhelm ? prm.p[0] : 1.0;
-    const double betd = CK ? prm.p[1] / prm.p[0] : 0.0;
-    const float2 bet2 = b2((float)betd);
-    // the orbits' offset factors: the first point of an orbit belongs to vertex 2
-    const double g0d = 1.0 - 3.0 * rule.x[0], g1d = 1.0 - 3.0 * rule.x[NQ6 / 2];
-    const float go[2] = {(float)g0d, (float)g1d};
-    const float2 g2 = f2(go[0], go[1]);
+    static_assert(!CK || SymTraits<K>::helm, "complex wavenumber: the Helmholtz kernels");
+    const double kap = mixed_kappa<K>(prm), g0d = mixed_g(rule, 0), g1d = mixed_g(rule, 1);
     const int tcount = (int)min((int64_t)rows, prm.ntest - t0);
     for (int idx = threadIdx.x; idx < tcount; idx += blockDim.x) {
         const int64_t t = prm.tsup[t0 + idx];
         Geom g;
         load_geom(prm.tg, prm.tne, t, prm.tnm ? (double)prm.tnm[t] : 1.0, g);
-        double e[3][3];
+        double e[3][3], m2 = 0.0;
         orbit_offsets(g, e);
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
 #pragma unroll
             for (int d = 0; d < 3; ++d) sb.e[idx][i][d] = (float)(kap * e[i][d]);
-            const double m = kap * kap * odot(e[i], e[i]);
+            const double ee = odot(e[i], e[i]), m = kap * kap * ee;
+            m2 = fmax(m2, ee);
             sb.hge[idx][0][i] = (float)(-0.5 * g0d * g0d * m);
             sb.hge[idx][1][i] = (float)(-0.5 * g1d * g1d * m);
             sb.c[idx][i] = __ldg(prm.tg + (22 + i) * prm.tne + t);
             sb.v[idx][i] = __ldg(prm.tel + 3 * t + i);
         }
-        sb.n[idx] = make_float4((float)g.n[0], (float)g.n[1], (float)g.n[2], 0.f);
+        sb.n[idx] = make_float4((float)g.n[0], (float)g.n[1], (float)g.n[2], (float)(MIXED_NEAR * kap * sqrt(m2)));
         sb.ie[idx] = g.ie;
     }
     __syncthreads();
 
     const int64_t si = tile_x * DP0_THREADS + threadIdx.x;
     if (si < prm.ntrial && t0 <= si) {
-    const int64_t s = prm.ssup[si];
-    Geom gs;
-    load_geom(prm.sg, prm.sne, s, prm.snm ? (double)prm.snm[s] : 1.0, gs);
-    const int sv0 = __ldg(prm.sel + 3 * s), sv1 = __ldg(prm.sel + 3 * s + 1), sv2 = __ldg(prm.sel + 3 * s + 2);
-    double sc[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) sc[d] = __ldg(prm.sg + (22 + d) * prm.sne + s);
-    float f[2][3];     // vertex offsets f_0, f_1 (f_2 = -f_0 - f_1)
-    float2 hgf[3];     // -g_q^2 |f_j|^2 / 2 of both orbits
-    {
-        double fd[3][3];
-        orbit_offsets(gs, fd);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const double m = -0.5 * kap * kap * odot(fd[j], fd[j]);
-            hgf[j] = f2((float)(g0d * g0d * m), (float)(g1d * g1d * m));
-        }
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            f[0][d] = (float)(kap * fd[0][d]);
-            f[1][d] = (float)(kap * fd[1][d]);
-        }
-    }
-    const float sn0 = (float)gs.n[0], sn1 = (float)gs.n[1], sn2 = (float)gs.n[2];
-    const double ek_r = (K == BEMPPCUDA_HELMHOLTZ_COMBINED) ? kap * prm.p[2] : kap;
-    const double ek_i = (K == BEMPPCUDA_HELMHOLTZ_COMBINED) ? kap * prm.p[3] : 0.0;
-    const double k2d = kap * kap;
-    // weights: w_b for the second test orbit, w_a / w_b applied in FP32 to the first; the trial orbits' at the end
-    const double wb = rule.w[NQ6 - 1];
-    const float2 rho2 = b2((float)(rule.w[0] / wb));
-    const float wqa = rule.wf[0], wqb = rule.wf[NQ6 - 1];
-    // centroid distances below near_r (scaled) may belong to vertex-sharing pairs
-    const double near2 = prm.near_r > 0.0 ? (kap * prm.near_r) * (kap * prm.near_r) : 1e300;
-    const auto fdot = [](const float a[3], float b0, float b1, float b2_) {
-        return fmaf(a[2], b2_, fmaf(a[1], b1, a[0] * b0));
-    };
-
-    for (int tt = 0; tt < tcount; ++tt) {
-        const int64_t row = t0 + tt;
-        if (row > si) break;
-        const double D0 = kap * (sc[0] - sb.c[tt][0]), D1 = kap * (sc[1] - sb.c[tt][1]),
-                     D2 = kap * (sc[2] - sb.c[tt][2]);
-        const double rc2 = fma(D2, D2, fma(D1, D1, D0 * D0));
-        const bool adj = row == si ||
-                         (prm.grids_identical && rc2 <= near2 && shares_vertex(sb.v[tt], sv0, sv1, sv2));
-        double a_re = 0.0, a_im = 0.0, b_re = 0.0, b_im = 0.0;  // A_ij, A_ji
-        if (!adj) {
-            const double rc = rc2 * rsqrt64(rc2);
-            float ph_s = 0.f, ph_c = 1.f;
-            if (ST::helm) phase_reduced32(rc, &ph_s, &ph_c);
-            // e^{-beta r_c'} (complex k), e^{-r_c'} (modified Helmholtz)
-            const double amp = CK ? exp_neg_reduced(betd * rc) : (ST::modhelm ? exp_neg_reduced(rc) : 1.0);
-            const float D0f = (float)D0, D1f = (float)D1, D2f = (float)D2, rcf = (float)rc;
-            const float2 rc_2 = b2(rcf), mrc_2 = b2(-rcf), mrc2_2 = b2(-(float)rc2);
-            // k (y - x).n_s = Dn - g_p e_i . n_s, one factor per test point; k (x - y).n_t = -Dt - g_q f_j . n_t,
-            // one per trial point
-            float Dn = 0.f;
-            float2 ynt[3];
-            if (ST::dlp_part) {
-                const float4 tn = sb.n[tt];
-                const float mDt = -fmaf(D2f, tn.z, fmaf(D1f, tn.y, D0f * tn.x));
-                const float m0 = -fdot(f[0], tn.x, tn.y, tn.z), m1 = -fdot(f[1], tn.x, tn.y, tn.z);
-                ynt[0] = fma2(b2(m0), g2, b2(mDt));
-                ynt[1] = fma2(b2(m1), g2, b2(mDt));
-                ynt[2] = fma2(b2(-(m0 + m1)), g2, b2(mDt));
-                Dn = fmaf(D2f, sn2, fmaf(D1f, sn1, D0f * sn0));
-            }
-            float2 hA[3];  // -A_q / 2
-            {
-                const float a0 = -fdot(f[0], D0f, D1f, D2f), a1 = -fdot(f[1], D0f, D1f, D2f);
-                hA[0] = fma2(b2(a0), g2, hgf[0]);
-                hA[1] = fma2(b2(a1), g2, hgf[1]);
-                hA[2] = fma2(b2(-(a0 + a1)), g2, hgf[2]);
-            }
-            float E[3][3], De[3], en[3];  // e_i . f_j, D . e_i, e_i . n_s
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const float e0 = sb.e[tt][i][0], e1 = sb.e[tt][i][1], e2 = sb.e[tt][i][2];
-                De[i] = fmaf(D2f, e2, fmaf(D1f, e1, D0f * e0));
-                if (ST::dlp_part) en[i] = fmaf(sn2, e2, fmaf(sn1, e1, sn0 * e0));
-                E[i][0] = fdot(f[0], e0, e1, e2);
-                E[i][1] = fdot(f[1], e0, e1, e2);
-                E[i][2] = -(E[i][0] + E[i][1]);
-            }
-            De[2] = -(De[0] + De[1]);
-            if (ST::dlp_part) en[2] = -(en[0] + en[1]);
-#pragma unroll
-            for (int j = 0; j < 3; ++j) E[2][j] = -(E[0][j] + E[1][j]);
-            float2 s0r = b2(0.f), s0m = b2(0.f), um = b2(0.f), ui = b2(0.f), vm = b2(0.f), vi = b2(0.f);
-#pragma unroll
-            for (int p = 0; p < NQ6; ++p) {
-                const int i = p % 3, op = p / 3;
-                if (p == NQ6 / 2) {  // second orbit: the first orbit's sums times w_a / w_b
-                    s0r = mul2(s0r, rho2);
-                    s0m = mul2(s0m, rho2);
-                    um = mul2(um, rho2);
-                    ui = mul2(ui, rho2);
-                    vm = mul2(vm, rho2);
-                    vi = mul2(vi, rho2);
-                }
-                const float2 hB = b2(fmaf(go[op], De[i], sb.hge[tt][op][i]));  // -B_p / 2
-                const float2 gp2 = f2(go[op] * go[0], go[op] * go[1]);
-                const float2 cp2 = b2(ST::dlp_part ? fmaf(-go[op], en[i], Dn) : 0.f);
-                float2 pum = b2(0.f), pui = b2(0.f);  // sums over q of the A_ij double-layer factors, times cp per p
-#pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    const float2 hs = fma2(b2(E[i][j]), gp2, add2(hA[j], hB));  // -s / 2
-                    const float2 mr2 = fma2(hs, b2(2.f), mrc2_2);              // -r'^2
-                    const float2 rinv = f2(rsqrt_approx(-mr2.x), rsqrt_approx(-mr2.y));
-                    // -theta
-                    float2 mt = b2(0.f);
-                    if (ST::helm || ST::modhelm) {
-                        const float2 t = fma2(mr2, rinv, rc_2);
-                        mt = fma2(fma2(t, fma2(t, b2(0.5f), mrc_2), hs), rinv, t);
-                    }
-                    if (!ST::helm) {
-                        // modified Helmholtz: e^{-theta} per pair (e^{-r_c'} per element pair), the double
-                        // layers' (1 + r') e^{-theta}
-                        float2 am = b2(1.f), am1 = b2(1.f);
-                        if (ST::modhelm) {
-                            am = f2(__expf(mt.x), __expf(mt.y));
-                            am1 = mul2(am, add2(b2(1.f), mul2(mul2(mr2, rinv), b2(-1.f))));
-                        }
-                        if (ST::slp_part) s0r = ST::modhelm ? fma2(rinv, am, s0r) : add2(rinv, s0r);
-                        if (ST::dlp_part) {
-                            float2 fr = mul2(mul2(rinv, rinv), rinv);
-                            if (ST::modhelm) fr = mul2(fr, am1);
-                            pum = add2(fr, pum);
-                            vm = fma2(fr, ynt[j], vm);
-                        }
-                    } else {
-                        float2 ms, cs;  // -sin, cos of theta
-                        sincos2_sym<PHC>(mt, &ms, &cs);
-                        if (CK) {
-                            const float2 am = f2(__expf(bet2.x * mt.x), __expf(bet2.x * mt.y));
-                            cs = mul2(cs, am);
-                            ms = mul2(ms, am);
-                        }
-                        if (ST::slp_part) {
-                            s0r = fma2(rinv, cs, s0r);
-                            s0m = fma2(rinv, ms, s0m);
-                        }
-                        if (ST::dlp_part) {
-                            const float2 fr = mul2(rinv, rinv);
-                            const float2 rb = CK ? add2(rinv, bet2) : rinv;  // 1 / r' (+ beta)
-                            const float2 mh1 = fma2(mul2(rb, b2(-1.f)), cs, ms);  // -h1
-                            const float2 h2 = fma2(rb, ms, cs);
-                            const float2 gt = mul2(fr, ynt[j]);
-                            pum = fma2(fr, mh1, pum);
-                            pui = fma2(fr, h2, pui);
-                            vm = fma2(gt, mh1, vm);
-                            vi = fma2(gt, h2, vi);
-                        }
+        MixedTrial tr;
+        load_trial_mixed<K>(prm, rule, si, tr);
+        // centroid distances below near_r (scaled) may belong to vertex-sharing pairs
+        const double near2 = prm.near_r > 0.0 ? (kap * prm.near_r) * (kap * prm.near_r) : 1e300;
+        sb.srad[threadIdx.x] = tr.rad;
+        for (int tt = 0; tt < tcount; ++tt) {
+            const int64_t row = t0 + tt;
+            if (row > si) break;
+            const double D0 = kap * (tr.c[0] - sb.c[tt][0]), D1 = kap * (tr.c[1] - sb.c[tt][1]),
+                         D2 = kap * (tr.c[2] - sb.c[tt][2]);
+            const double rc2 = fma(D2, D2, fma(D1, D1, D0 * D0));
+            const bool adj = row == si || (prm.grids_identical && rc2 <= near2 &&
+                                           shares_vertex(sb.v[tt], tr.v[0], tr.v[1], tr.v[2]));
+            double a_re = 0.0, a_im = 0.0, b_re = 0.0, b_im = 0.0;  // A_ij, A_ji
+            if (!adj) {
+                mixed_pair<K, PHC, CK, false>(prm, rule, sb, tt, tr, D0, D1, D2, rc2, a_re, a_im, b_re, b_im);
+                if (rc2 <= near2) {
+                    const float rs = sb.n[tt].w + sb.srad[threadIdx.x];
+                    if ((float)rc2 < rs * rs) {  // in place of what the expanded square gave
+                        double ab[4];
+                        mixed_near_pair<K, PHC, CK>(prm, rule, sb, tt, si, ab);
+                        a_re = ab[0];
+                        a_im = ab[1];
+                        b_re = ab[2];
+                        b_im = ab[3];
                     }
                 }
-                if (ST::dlp_part) {
-                    um = fma2(cp2, pum, um);
-                    if (ST::helm) ui = fma2(cp2, pui, ui);
-                }
             }
-            // entry = w_b [kappa eta S0 + kappa^2 (-h1 sum + i h2 sum)], rotated by exp(i r_c') and scaled; um and vm
-            // hold the -h1 sums (Helmholtz) or the sums of w (d'.n) / r'^3 (real kernels)
-            const auto orbits = [&](float2 v) { return (double)fmaf(wqa, v.x, wqb * v.y); };
-            double sr = 0.0, sim = 0.0;
-            if (ST::slp_part) {
-                const double xr = orbits(s0r), xi = ST::helm ? -orbits(s0m) : 0.0;
-                sr = fma(ek_r, xr, -ek_i * xi);
-                sim = fma(ek_r, xi, ek_i * xr);
-            }
-            double dr = 0.0, di = 0.0, er = 0.0, ei = 0.0;
-            if (ST::dlp_part) {
-                const double sg = ST::helm ? k2d : -k2d;
-                dr = sg * orbits(um);
-                er = sg * orbits(vm);
-                if (ST::helm) {
-                    di = k2d * orbits(ui);
-                    ei = k2d * orbits(vi);
-                }
-            }
-            if (ST::swap) {
-                a_re = er;
-                a_im = ei;
-                b_re = dr;
-                b_im = di;
-            } else {
-                a_re = sr + dr;
-                a_im = sim + di;
-                b_re = sr + er;
-                b_im = sim + ei;
-            }
-            const double scale = BC_INV_4PI * sb.ie[tt] * gs.ie * wb * amp;
-            const double pc = (double)ph_c, ps = (double)ph_s;
-            double tr = a_re * pc - a_im * ps;
-            a_im = (a_re * ps + a_im * pc) * scale;
-            a_re = tr * scale;
-            tr = b_re * pc - b_im * ps;
-            b_im = (b_re * ps + b_im * pc) * scale;
-            b_re = tr * scale;
+            store_pair<STRIPE>(prm, row, si, adj, a_re, a_im, b_re, b_im);
         }
-        store_pair<STRIPE>(prm, row, si, adj, a_re, a_im, b_re, b_im);
-    }
     }
     __syncthreads();
 }

@@ -10,7 +10,8 @@
 //   s = r'^2 - r_c'^2 = A_q + B_p - 2 g_p g_q e_i . f_j
 // is formed in FP32, 1/r' by rsqrt.approx, the phase offset theta = r' - r_c'
 // by one Newton step on theta^2 + 2 r_c' theta = s (dp0_sym.cuh) and its sine /
-// cosine by the fitted FP32 polynomials.  The trial points of one vertex, one
+// cosine by the fitted FP32 polynomials; near pairs difference the coordinates
+// (near_mr2, dp0.cuh) and follow the sweep.  The trial points of one vertex, one
 // of each orbit, travel together through packed f32x2 FMAs; the blocks of the
 // trial sums T_j(p) = sum_q w_q psi_j(q) K add real and imaginary parts packed.
 // Double layers: with h = (i r' - 1) exp(i theta) / r'^3 and d' = k (y - x),
@@ -64,6 +65,8 @@
 // the DP0 sweep; error 3.74e-8 either way.
 #pragma once
 
+#include <type_traits>
+
 #include "p1.cuh"
 #include "rwg.cuh"
 #include "warp_cols.cuh"
@@ -79,6 +82,7 @@ struct TestBlockP1m {
     double mult[P1_TCHUNK][3];
     int64_t row[P1_TCHUNK][3];
     int v[P1_TCHUNK][3];
+    float rad[P1_TCHUNK];  // MIXED_NEAR R
 };
 
 // NT, NS: test / trial functions per element, 3 (P1, DP1, RWG / SNC) or 1 (a P0 space beside a P1 one: its
@@ -128,16 +132,18 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, O
         double c[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) c[d] = __ldg(prm.tg + (22 + d) * prm.tne + t);
-        double eo[3][3];
+        double eo[3][3], m2 = 0.0;
         orbit_offsets(g, eo);
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
 #pragma unroll
             for (int d = 0; d < 3; ++d) sb.e[idx][i][d] = (float)(kap * eo[i][d]);
-            const double m = -0.5 * kap * kap * odot(eo[i], eo[i]);
+            const double ee = odot(eo[i], eo[i]), m = -0.5 * kap * kap * ee;
+            m2 = fmax(m2, ee);
             sb.hge[idx][0][i] = (float)(oc.gg[0] * m);
             sb.hge[idx][1][i] = (float)(oc.gg[1] * m);
         }
+        sb.rad[idx] = (float)(MIXED_NEAR * kap * sqrt(m2));
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             sb.c[idx][d] = c[d];
@@ -182,12 +188,14 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, O
     // vertex offsets f_0, f_1 (f_2 = -f_0 - f_1) and -g_q^2 |f_j|^2 / 2 of both orbits
     float f[2][3];
     float2 hgf[3];
+    float srad;  // MIXED_NEAR R
     {
-        double fd[3][3];
+        double fd[3][3], m2 = 0.0;
         orbit_offsets(gs, fd);
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            const double m = -0.5 * kap * kap * odot(fd[j], fd[j]);
+            const double ff = odot(fd[j], fd[j]), m = -0.5 * kap * kap * ff;
+            m2 = fmax(m2, ff);
             hgf[j] = f2((float)(oc.gg[0] * m), (float)(oc.gg[1] * m));
         }
 #pragma unroll
@@ -195,6 +203,7 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, O
             f[0][d] = (float)(kap * fd[0][d]);
             f[1][d] = (float)(kap * fd[1][d]);
         }
+        srad = (float)(MIXED_NEAR * kap * sqrt(m2));
     }
     // orbit constants in FP32: offsets g, and w times the linear functions at a point: the own vertex's (c + d) and
     // the other two's (d).  (c and d times the orbit's sum, as in FP64, would cancel: c < 0 in the first orbit.)
@@ -228,10 +237,10 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, O
     double2(&st)[3][WC_SLOTS] = sst[warp];
     double2(&st_t)[3][SKEW ? WC_SLOTS : 1] = sst_t[SKEW ? warp : 0];
 
-    for (int tt = 0; tt < tcount; ++tt) {
-        const bool done = !active || (SYM && t0 + tt >= si);  // rows increase with tt
-        if (__all_sync(0xffffffffu, done)) break;
-        if (done || (prm.grids_identical && shares_vertex(sb.v[tt], sv0, sv1, sv2))) {
+    // one test element: the blocks of the warp's pairs (has: this lane has one), staged and added per column
+    const auto row = [&](int tt, bool has, double D0, double D1, double D2, auto near_) {
+        constexpr bool NEAR = decltype(near_)::value;
+        if (!has) {
             // no pair: zeros in this lane's staging positions
 #pragma unroll
             for (int i = 0; i < NT; ++i)
@@ -242,8 +251,6 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, O
                         if (SKEW) st_t[i][pos[j]] = make_double2(0.0, 0.0);
                     }
         } else {
-        const double D0 = kap * (sc[0] - sb.c[tt][0]), D1 = kap * (sc[1] - sb.c[tt][1]),
-                     D2 = kap * (sc[2] - sb.c[tt][2]);
         const double rc2 = fma(D2, D2, fma(D1, D1, D0 * D0));
         const double rc = sqrt(rc2);
         // the element pair's factor: exp(i r_c'), times exp(-beta r_c') (complex k); exp(-r_c') (modified)
@@ -259,13 +266,6 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, O
         const float D0f = (float)D0, D1f = (float)D1, D2f = (float)D2;
         const float rcf = (float)rc;
         const float2 rc_2 = b2(rcf), mrc_2 = b2(-rcf), mrc2_2 = b2(-(float)rc2);
-        float2 hA[3];  // -A_q / 2
-        {
-            const float a0 = -fdot(f[0], D0f, D1f, D2f), a1 = -fdot(f[1], D0f, D1f, D2f);
-            hA[0] = fma2(b2(a0), g2, hgf[0]);
-            hA[1] = fma2(b2(a1), g2, hgf[1]);
-            hA[2] = fma2(b2(-(a0 + a1)), g2, hgf[2]);
-        }
         // normal terms: D . n_s; -(d'.n_t) = -(D . n_t) - g_q f_j . n_t per trial point
         const float Dns = NS_SUM ? fmaf(D2f, sn2, fmaf(D1f, sn1, D0f * sn0)) : 0.f;
         float2 cm[3] = {b2(0.f), b2(0.f), b2(0.f)};
@@ -277,43 +277,73 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, O
             cm[1] = fma2(b2(m1), g2, mDt);
             cm[2] = fma2(b2(-(m0 + m1)), g2, mDt);
         }
-        float E[3][3], De[3], en[3] = {0.f, 0.f, 0.f};  // e_i . f_j, D . e_i, e_i . n_s
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const float e0 = sb.e[tt][i][0], e1 = sb.e[tt][i][1], e2 = sb.e[tt][i][2];
-            De[i] = fmaf(D2f, e2, fmaf(D1f, e1, D0f * e0));
-            if (NS_SUM) en[i] = fmaf(sn2, e2, fmaf(sn1, e1, sn0 * e0));
-            E[i][0] = fdot(f[0], e0, e1, e2);
-            E[i][1] = fdot(f[1], e0, e1, e2);
-            E[i][2] = -(E[i][0] + E[i][1]);
-        }
-        De[2] = -(De[0] + De[1]);
-        if (NS_SUM) en[2] = -(en[0] + en[1]);
-#pragma unroll
-        for (int j = 0; j < 3; ++j) E[2][j] = -(E[0][j] + E[1][j]);
         // (re, im) blocks: the block of (i, j): single layer, or its double layer; SKEW: the transposed pair's
         float2 l[NT][NS], u[SKEW ? NT : 1][SKEW ? NS : 1];
         const auto axpy = [](float a, float2 x, float2 y) -> float2 {
             return REAL ? f2(fmaf(a, x.x, y.x), 0.f) : fma2(b2(a), x, y);
         };
 #pragma unroll
+        for (int a = 0; a < NT; ++a)
+#pragma unroll
+            for (int j = 0; j < NS; ++j) {
+                l[a][j] = b2(0.f);
+                if (SKEW) u[a % (SKEW ? NT : 1)][j % (SKEW ? NS : 1)] = b2(0.f);
+            }
+        float2 hA[3];  // -A_q / 2
+        if (!NEAR) {
+            const float a0 = -fdot(f[0], D0f, D1f, D2f), a1 = -fdot(f[1], D0f, D1f, D2f);
+            hA[0] = fma2(b2(a0), g2, hgf[0]);
+            hA[1] = fma2(b2(a1), g2, hgf[1]);
+            hA[2] = fma2(b2(-(a0 + a1)), g2, hgf[2]);
+        }
+        float E[3][3], De[3], en[3] = {0.f, 0.f, 0.f};  // e_i . f_j, D . e_i, e_i . n_s
+        if (!NEAR) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const float e0 = sb.e[tt][i][0], e1 = sb.e[tt][i][1], e2 = sb.e[tt][i][2];
+                De[i] = fmaf(D2f, e2, fmaf(D1f, e1, D0f * e0));
+                if (NS_SUM) en[i] = fmaf(sn2, e2, fmaf(sn1, e1, sn0 * e0));
+                E[i][0] = fdot(f[0], e0, e1, e2);
+                E[i][1] = fdot(f[1], e0, e1, e2);
+                E[i][2] = -(E[i][0] + E[i][1]);
+            }
+            De[2] = -(De[0] + De[1]);
+            if (NS_SUM) en[2] = -(en[0] + en[1]);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) E[2][j] = -(E[0][j] + E[1][j]);
+        }
+#pragma unroll (NEAR ? 1 : NQ6)
         for (int p = 0; p < NQ6; ++p) {
             const int i = p % 3, op = p / 3;
-            const float2 hB = b2(fmaf(go[op], De[i], sb.hge[tt][op][i]));  // -B_p / 2
-            const float2 gp2 = f2(go[op] * go[0], go[op] * go[1]);
+            const float gp = op == 0 ? go[0] : go[1];
+            float x[3];  // NEAR: D - g_p e_i
+            float2 hB, gp2;
+            if (NEAR) {
+                x[0] = fmaf(-gp, sb.e[tt][i][0], D0f);
+                x[1] = fmaf(-gp, sb.e[tt][i][1], D1f);
+                x[2] = fmaf(-gp, sb.e[tt][i][2], D2f);
+            } else {
+                hB = b2(fmaf(gp, De[i], sb.hge[tt][op][i]));  // -B_p / 2
+                gp2 = f2(gp * go[0], gp * go[1]);
+            }
             float2 kr[3], ki[3];
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
-                const float2 hs = fma2(b2(E[i][j]), gp2, add2(hA[j], hB));  // -s / 2
-                const float2 mr2 = fma2(hs, b2(2.f), mrc2_2);              // -r'^2
+                float2 hs, mr2;  // -s / 2, -r'^2
+                if (NEAR) {
+                    mr2 = near_mr2(x, f, j, g2);
+                } else {
+                    hs = fma2(b2(E[i][j]), gp2, add2(hA[j], hB));
+                    mr2 = fma2(hs, b2(2.f), mrc2_2);
+                }
                 const float2 rinv = f2(rsqrt_approx(-mr2.x), rsqrt_approx(-mr2.y));
                 const float2 mrp = mul2(mr2, rinv);  // -r'
                 // cs - i ms: exp(i theta) (Helmholtz), times exp(-beta theta) (complex k); exp(-theta)
                 // (modified, ms = 0); 1 (Laplace)
                 float2 ms = b2(0.f), cs = b2(1.f);
                 if (!LAP) {
-                    const float2 t = fma2(mr2, rinv, rc_2);
-                    const float2 mt = fma2(fma2(t, fma2(t, b2(0.5f), mrc_2), hs), rinv, t);  // -theta
+                    float2 mt = fma2(mr2, rinv, rc_2);  // -theta
+                    if (!NEAR) mt = fma2(fma2(mt, fma2(mt, b2(0.5f), mrc_2), hs), rinv, mt);
                     if (!MH) sincos2<PHC>(mt, &ms, &cs);
                     if (MH || CK) {
                         const float2 am = f2(__expf(bet * mt.x), __expf(bet * mt.y));
@@ -370,16 +400,18 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, O
                 for (int j = 0; j < NS; ++j) V[j] = f2(sums(vr, j), REAL ? 0.f : sums(vi, j));
             }
             // into the blocks: (i, j) double layer -> T times d'.n_s, adjoint -> V; SKEW: the other one at (j, i)
-            const float dns = NS_SUM ? fmaf(-go[op], en[i], Dns) : 1.f;
+            const float dns = !NS_SUM ? 1.f : NEAR ? fdot(x, sn0, sn1, sn2) : fmaf(-gp, en[i], Dns);
 #pragma unroll
             for (int a = 0; a < NT; ++a) {
-                const float w = NT == 1 ? wp_[op] : a == i ? own_[op] : oth_[op], wn = NS_SUM ? w * dns : w;
+                const float w = op == 0 ? (NT == 1 ? wp_[0] : a == i ? own_[0] : oth_[0])
+                                        : (NT == 1 ? wp_[1] : a == i ? own_[1] : oth_[1]);
+                const float wn = NS_SUM ? w * dns : w;
 #pragma unroll
                 for (int j = 0; j < NS; ++j) {
-                    l[a][j] = axpy(DL ? wn : w, AD ? V[j] : T[j], p == 0 ? b2(0.f) : l[a][j]);
+                    l[a][j] = axpy(DL ? wn : w, AD ? V[j] : T[j], l[a][j]);
                     if (SKEW) {
                         constexpr int A_ = SKEW ? NT : 1, B_ = SKEW ? NS : 1;
-                        u[a % A_][j % B_] = axpy(DL ? w : wn, DL ? V[j] : T[j], p == 0 ? b2(0.f) : u[a % A_][j % B_]);
+                        u[a % A_][j % B_] = axpy(DL ? w : wn, DL ? V[j] : T[j], u[a % A_][j % B_]);
                     }
                 }
             }
@@ -562,6 +594,27 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_mixed(RegParams prm, O
             }
         }
         __syncwarp();  // the staging arrays are rewritten by the next test element
+    };
+
+    static_assert(P1_TCHUNK <= 32, "a bit per row");
+    uint32_t near_rows = 0;  // left for after the sweep, whose registers and schedule stay its own
+    for (int tt = 0; tt < tcount; ++tt) {
+        const bool done = !active || (SYM && t0 + tt >= si);  // rows increase with tt
+        if (__all_sync(0xffffffffu, done)) break;
+        bool has = !done && !(prm.grids_identical && shares_vertex(sb.v[tt], sv0, sv1, sv2));
+        const double D0 = kap * (sc[0] - sb.c[tt][0]), D1 = kap * (sc[1] - sb.c[tt][1]),
+                     D2 = kap * (sc[2] - sb.c[tt][2]);
+        const float rs = sb.rad[tt] + srad;
+        if (has && (float)fma(D2, D2, fma(D1, D1, D0 * D0)) < rs * rs) {
+            near_rows |= 1u << tt;
+            has = false;
+        }
+        row(tt, has, D0, D1, D2, std::false_type());
+    }
+    for (uint32_t rows_ = __reduce_or_sync(0xffffffffu, near_rows); rows_ != 0; rows_ &= rows_ - 1) {
+        const int tt = __ffs(rows_) - 1;
+        row(tt, (near_rows >> tt) & 1u, kap * (sc[0] - sb.c[tt][0]), kap * (sc[1] - sb.c[tt][1]),
+            kap * (sc[2] - sb.c[tt][2]), std::true_type());
     }
 }
 

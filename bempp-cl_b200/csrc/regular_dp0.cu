@@ -25,9 +25,9 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_dp0_fp64_sym(RegParams pr
 #endif
 
 template <int K, int PHC, bool STRIPE = false, bool CK = false>
-__global__ void __launch_bounds__(DP0_THREADS, BC_MSYM_MIN_BLOCKS) regular_dp0_mixed_sym(RegParams prm, QuadRule rule,
-                                                                                      int64_t row0, int64_t row1,
-                                                                                      int tile_rows) {
+__global__ void __launch_bounds__(DP0_THREADS, BC_MSYM_MIN_BLOCKS)
+    regular_dp0_mixed_sym(const __grid_constant__ RegParams prm, const __grid_constant__ QuadRule rule, int64_t row0,
+                          int64_t row1, int tile_rows) {
     const int64_t t0 = row0 + (int64_t)blockIdx.y * tile_rows;
     if (t0 >= ((int64_t)blockIdx.x + 1) * DP0_THREADS) return;
     __shared__ TestBlock32q sb;

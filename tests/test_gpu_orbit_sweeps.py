@@ -182,3 +182,26 @@ def test_nearly_imaginary_wavenumber(oracle, name, k):
     from bempp_cuda.shapes import ellipsoid
 
     _check(oracle, ("helmholtz", name, "DP", 0), ellipsoid(2, 1.0, 0.8, 1.2), k, 1e-12)
+
+
+STRETCHED = {"flat": lambda: _ellipsoid(1.0, 1.0, 0.01), "thin": lambda: _ellipsoid(1.0, 0.03, 0.03),
+             "sheets": lambda: _sheets(1e-2), "crossing": lambda: _united(_octahedron(), _midpoint_refined(_octahedron()))}
+
+
+def _ellipsoid(a, b, c):
+    from bempp_cuda.shapes import ellipsoid
+
+    return ellipsoid(3, a, b, c)
+
+
+@pytest.mark.parametrize("mesh", list(STRETCHED))
+@pytest.mark.parametrize("case", OPERATORS)
+def test_mixed_with_near_elements(oracle, case, mesh):
+    """Elements that share no vertex and lie closer than their size: distances by differenced coordinates, which lose
+    size / distance of FP32's digits where the expanded square loses its square.  1e-6 as elsewhere; the crossing
+    triangulations lie in one plane, their points 0.02 apart at a size of 1.4, so the double layers' normal terms are
+    6e-8 * 70 = 4e-6 of their distances instead of zero."""
+    grid = STRETCHED[mesh]()
+    tol = 4e-6 if mesh == "crossing" else 1e-6
+    for k in (1.3,) if case[0] in ("laplace", "modified_helmholtz") else (1.3, 6.0, 1.3 + 0.5j):
+        _check(oracle, case, grid, k, tol, device_interface="cuda_mixed")
