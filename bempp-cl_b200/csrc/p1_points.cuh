@@ -36,8 +36,8 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_points(RegParams prm, 
     constexpr bool HYP = ASM == BEMPPCUDA_ASM_LAPLACE_HYP;
     constexpr bool HELM = (K == BEMPPCUDA_HELMHOLTZ_SLP || K == BEMPPCUDA_HELMHOLTZ_DLP ||
                            K == BEMPPCUDA_HELMHOLTZ_ADLP);
-    constexpr bool DL = K == BEMPPCUDA_LAPLACE_DLP || K == BEMPPCUDA_HELMHOLTZ_DLP;
-    constexpr bool AD = K == BEMPPCUDA_LAPLACE_ADLP || K == BEMPPCUDA_HELMHOLTZ_ADLP;
+    constexpr bool DL = K == BEMPPCUDA_HELMHOLTZ_DLP, AD = K == BEMPPCUDA_HELMHOLTZ_ADLP;
+    static_assert(HELM || K == BEMPPCUDA_LAPLACE_SLP, "the operators of p1_points_form");
     constexpr bool PH = HELM && CLS > 0;
     static_assert(!SYM || NT == NS, "the symmetric sweep needs one space on both sides");
     constexpr bool SKEW = SYM && (DL || AD);  // the transposed block uses the other element's normal
@@ -157,47 +157,30 @@ __global__ void __launch_bounds__(DP0_THREADS) regular_p1_points(RegParams prm, 
                 const double rinv = rsqrt64(r2);
                 double kre, kim = 0.0;  // kernel value without 1/(4 pi)
                 double k2re = 0.0, k2im = 0.0;  // SKEW: the transposed pair's kernel
-                if (SKEW) {
-                    double hre, him;  // double layer of trial normal n: (dot with n) (hre + i him)
-                    if (!HELM) {
-                        hre = -rinv * rinv * rinv;
-                        him = 0.0;
-                    } else {
-                        const double r = r2 * rinv;
-                        double sn, cs;
-                        sincos_off64<CLS>(fma(kr, r, -krc), &sn, &cs);
-                        const double rinv2 = rinv * rinv, rk = rinv;
-                        hre = -rinv2 * fma(rk, cs, kr * sn);
-                        him = rinv2 * fma(kr, cs, -rk * sn);
-                    }
-                    // h alone (its trial-normal factor xn is applied per test point), and h times the
-                    // test-normal factor of this trial point
-                    kre = hre;
-                    kim = him;
-                    k2re = mdt[q % (SKEW ? NQ6 : 1)] * hre;
-                    k2im = mdt[q % (SKEW ? NQ6 : 1)] * him;
-                } else if (!HELM) {
-                    if (K == BEMPPCUDA_LAPLACE_SLP) {
-                        kre = rinv;
-                    } else {
-                        const double dot = DL ? ynv[q] + xn
-                                              : fma(d2, sb.n[tt][2], fma(d1, sb.n[tt][1], d0 * sb.n[tt][0]));
-                        kre = (DL ? -dot : dot) * rinv * rinv * rinv;
-                    }
+                if (!HELM) {
+                    kre = rinv;
                 } else {
                     const double r = r2 * rinv;
                     double sn, cs;
                     sincos_off64<CLS>(fma(kr, r, -krc), &sn, &cs);
-                    if (K == BEMPPCUDA_HELMHOLTZ_SLP) {
+                    if (SKEW) {
+                        // double layer of trial normal n: (dot with n) (kre + i kim), whose trial-normal factor xn is
+                        // applied per test point, and the same times the test-normal factor of this trial point
+                        const double rinv2 = rinv * rinv;
+                        kre = -rinv2 * fma(rinv, cs, kr * sn);
+                        kim = rinv2 * fma(kr, cs, -rinv * sn);
+                        k2re = mdt[q % (SKEW ? NQ6 : 1)] * kre;
+                        k2im = mdt[q % (SKEW ? NQ6 : 1)] * kim;
+                    } else if (K == BEMPPCUDA_HELMHOLTZ_SLP) {
                         kre = cs * rinv;
                         kim = sn * rinv;
                     } else {
                         // (ikr - 1) e^{ikr} dot / r^3 = g (-h1 + i h2), g = dot / r^2
                         const double dot = DL ? ynv[q] + xn
                                               : -fma(d2, sb.n[tt][2], fma(d1, sb.n[tt][1], d0 * sb.n[tt][0]));
-                        const double g = dot * rinv * rinv, rk = rinv;
-                        kre = -g * fma(rk, cs, kr * sn);
-                        kim = g * fma(kr, cs, -rk * sn);
+                        const double g = dot * rinv * rinv;
+                        kre = -g * fma(rinv, cs, kr * sn);
+                        kim = g * fma(kr, cs, -rinv * sn);
                     }
                 }
 #pragma unroll
