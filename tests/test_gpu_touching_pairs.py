@@ -3,7 +3,7 @@ bemppcuda_assemble_singular on the same pairs (B200).
 
 Every operator, real and complex wavenumbers in the offset classes 2, 1 and 0, meshes whose pairs take a warp each
 (32 elements) and eight lanes each (2048), a space on part of the grid, and both vertex-adjacent orders with and without
-mirroring.  The two differ in the order of 512 - 1536 terms: 1e-13 of the matrix norm.  The normal terms of the double
+mirroring; blocks into the caller's array; other orders, which take the tables, against the oracle.  The two differ in the order of 512 - 1536 terms: 1e-13 of the matrix norm.  The normal terms of the double
 layers and the triple products of the magnetic field cancel between neighbours: the tables difference coordinates,
 eps / h (2e-15 of the element size h = 0.06 at 2048 elements), and the result is smaller than the terms by the angle
 between neighbours, about h, so each term carries 3e-14 and entries of neighbouring signs more: 1e-12.
@@ -11,6 +11,8 @@ between neighbours, about h, so each term carries 3e-14 and entries of neighbour
 
 import numpy as np
 import pytest
+
+from conftest import rel_fro
 
 pytestmark = pytest.mark.gpu
 
@@ -103,19 +105,64 @@ def test_coincident_double_layer_is_zero():
     assert float(a.diagonal().abs().max()) == 0.0
 
 
-@pytest.mark.parametrize("order", [3, 4])
-def test_other_orders_take_the_tables(order, monkeypatch):
-    """A singular order other than 4 goes through the flat tables; both orders agree to their quadrature error."""
+@pytest.mark.parametrize("order", [3, 5])
+@pytest.mark.parametrize("case", [("laplace", "single_layer", "DP", 0), ("helmholtz", "double_layer", "DP", 0),
+                                  ("helmholtz", "single_layer", "P", 1), ("laplace", "hypersingular", "P", 1)])
+def test_other_orders_take_the_tables(oracle, case, order):
+    """A singular order other than 4 goes through the flat tables, vertex-adjacent pairs once for both orders or each on
+    its own: against the oracle at that order, 1e-12 as the other FP64 paths."""
+    from bempp_cuda import operators
+    from bempp_cuda.assembly import result_dtype, singular_into_dense
+    from bempp_cuda.shapes import ellipsoid
+    from bempp_cuda.space import function_space
+    from cases import oracle_dense
+
+    equation, name, kind, degree = case
+    space = function_space(ellipsoid(2, 1.0, 0.8, 1.2), kind, degree)
+    parameters = operators.Parameters()
+    parameters.quadrature.singular = order
+    factory = getattr(getattr(operators.boundary, equation), name)
+    op = factory(space, space, space, *(() if equation == "laplace" else (1.5,)), parameters=parameters)
+    ref = oracle_dense(oracle, op, space, space)
+    assert rel_fro(op.weak_form().A, ref) < 1e-12
+    parts = []
+    for mirror in (True, False):
+        out = torch.zeros(ref.shape, dtype=result_dtype(op.descriptor), device="cuda")
+        parts.append(singular_into_dense(out, op.descriptor, space, space, parameters, mirror=mirror))
+    assert float(torch.linalg.vector_norm(parts[0] - parts[1]) / np.linalg.norm(ref)) < 1e-12
+
+
+@pytest.mark.parametrize("equation,name,kind,degree", [CASES[1], CASES[5], CASES[8], CASES[12], CASES[13]])
+def test_values_per_pair(equation, name, kind, degree):
+    """The pairs' blocks in the caller's array instead of a matrix, added to what is there."""
     from bempp_cuda import _lib, operators
+    from bempp_cuda.assembly import _set_params, kernel_ids, result_dtype
+    from bempp_cuda.device import current_stream, device_grid, device_singular_rule, device_space
     from bempp_cuda.shapes import ellipsoid
     from bempp_cuda.space import function_space
 
-    space = function_space(ellipsoid(2, 1.0, 0.8, 1.2), "P", 1)
-    parameters = operators.Parameters()
-    parameters.quadrature.singular = order
-    op = operators.boundary.helmholtz.single_layer(space, space, space, 1.5, parameters=parameters)
-    got = op.weak_form().tensor
-    lib = _lib.load()
-    monkeypatch.setattr(_lib, "load", lambda: _Library(lib))
-    ref = operators.boundary.helmholtz.single_layer(space, space, space, 1.5, parameters=parameters).weak_form().tensor
-    assert float(torch.linalg.vector_norm(got - ref) / torch.linalg.vector_norm(ref)) < 1e-13
+    grid = ellipsoid(2, 1.0, 0.8, 1.2)
+    domain = function_space(grid, kind, degree)
+    dual = function_space(grid, "SNC", 0) if kind == "RWG" else domain
+    d = _descriptor(equation, name, domain, dual, 1.5)
+    rule = device_singular_rule(grid, 4, dual.support, domain.support)
+    shapes = device_space(dual).nshape * device_space(domain).nshape
+    lib, out = _lib.load(), []
+    for entry in (lambda a: lib.bemppcuda_assemble_singular_duffy(a, 4, current_stream()),
+                  lambda a: lib.bemppcuda_assemble_singular(a, current_stream())):
+        args = _lib.SingularArgs()
+        args.kernel, args.assembly = kernel_ids(d)
+        args.is_complex = 1 if d.is_complex else 0
+        _set_params(args, d.options)
+        args.grid, args.test, args.trial = (device_grid(grid).record(), device_space(dual).record(),
+                                            device_space(domain).record())
+        rule.fill(args)
+        args.phase_radius = 1.0001 * 2.0 * device_grid(grid).radius
+        values = torch.ones(rule.npairs * shapes, dtype=result_dtype(d), device="cuda")
+        args.values = values.data_ptr()
+        _lib.check(entry(args))
+        out.append(values - 1.0)
+    assert float(torch.linalg.vector_norm(out[1])) > 0.0
+    tol = 1e-12 if "double" in name or name == "magnetic_field" else 1e-13
+    # (adding to one loses eps per value)
+    assert float((out[0] - out[1]).abs().max()) < tol * float(out[1].abs().max()) + 4e-16
