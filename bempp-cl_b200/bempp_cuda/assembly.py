@@ -282,9 +282,11 @@ def singular_into_dense(result, descriptor, domain, dual_to_range, parameters, d
 
     ``rows=(lo, hi)``: only the pairs whose test element is one of the support
     elements lo .. hi-1 of ``dual_to_range`` (support in increasing order).
-    ``mirror`` (default) lets the DP0 kernel evaluate each vertex-adjacent pair
-    once for both orders when both spaces are the same; ``mirror=False``
-    evaluates every ordered pair on its own.
+    ``mirror`` (default) lets each vertex-adjacent pair be evaluated once for
+    both orders when both spaces are the same, or (Maxwell) have equal supports
+    and dof maps: every operator at singular order 4, at other orders the DP0
+    operators and the P1 single layers and hypersingular operators;
+    ``mirror=False`` evaluates every ordered pair on its own.
     """
     kernel, assembly = kernel_ids(descriptor)
     if result.numel() == 0:

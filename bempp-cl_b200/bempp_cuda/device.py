@@ -27,7 +27,8 @@ _CACHE_ATTR = "_bempp_cuda_device_cache"
 
 # A small operator's call is bound by the host (128 elements: 18 us on the device), so what a call looks up here is kept
 # short: one device lookup per call handed on as ``dev``, records built with the device copies that they point into,
-# the raw stream handle without a Stream object, no availability query once CUDA is initialised.
+# the raw stream handle without a Stream object (the lookup inside torch.cuda.current_stream, which has no public name),
+# no availability query once CUDA is initialised.
 
 
 def require_cuda():

@@ -42,7 +42,7 @@ struct SymTraits {
 //    centroid distance by offset class (fastmath.cuh), a complex one or exp(-w r) reduced per point pair.
 //  orbit: the two-orbit rule (orbit_pair.cuh), where the amplitudes exp(-Im k r) and exp(-w r) are factored too.
 // The orbit form takes fewer FP64 operations in every kernel, but its chains depend on each other more and it
-// runs the FP64 pipe at 73 - 78 % against 82 - 86 %: with the amplitudes' library exponential gone it is
+// runs the FP64 pipe at 75 - 80 % against 86 %: with the amplitudes' library exponential gone it is
 // 1.25 - 1.6 times faster (n = 16200: combined field k = 4 + 0.4i 28.5 -> 17.5 ms, modified Helmholtz single
 // layer 11.2 -> 8.9 ms), without them between 0.92 (Laplace single layer) and 1.05 of the points form (double layer).
 constexpr int SYM_POINTS = 0, SYM_POINTS_CK = 3, SYM_ORBIT = 4, SYM_ORBIT_CK = 8;
@@ -721,8 +721,9 @@ __device__ __noinline__ void mixed_near_pair(const RegParams &prm, const QuadRul
 // the pair phase exp(i r_c') by phase_reduced32.  The FP32 sums of the
 // first test orbit are scaled by w_a / w_b when the second begins, and everything is converted to FP64 once,
 // times w_b.
-// Bound by the FMA pipe with the special-function unit close behind.  Combined field, 32768 elements, k = 10: 22.02 ->
-// 21.12 ms (against pairs of neighbouring trial points and the reciprocal), error 1.4e-8 either way.
+// Bound by the FMA pipe: 68 % of its cycles, the special-function unit 49 %, issue 55 %, the first stall its throttle.
+// Combined field, 32768 elements, k = 10: 22.02 -> 21.09 ms (against pairs of neighbouring trial points and the
+// reciprocal), error 1.4e-8 either way.
 // CK: a complex wavenumber k = kr + i ki in units of 1/kr: the amplitude e^{-beta r'} (beta = ki / kr)
 // split like the phase, e^{-beta theta} per point pair by __expf and e^{-beta r_c'} per element pair by
 // exp_neg_reduced; the double-layer factor (i k r - 1) = -(1 + beta r') + i r' turns 1 / r' into

@@ -25,8 +25,8 @@
 // layer: the double layer of the transposed pair (test j, trial i) is the
 // adjoint double layer of (i, j), so both blocks share the values of
 // H = (ikr - 1) e^{ikr} / r^3 and differ in the normal factor.
-// Bound by the FP64 pipe (73 - 80 %; an FMA of three unshared registers issues at
-// 72 % of its peak).  8192 elements, points form before -> orbit form:
+// Bound by the FP64 pipe (69 % in the hypersingular sweep, 72 % in the single layer with
+// a complex wavenumber; an FMA of three unshared registers issues at 72 % of its peak).  8192 elements, points form before -> orbit form:
 // Helmholtz hypersingular k = 5 4.27 -> 4.05 ms, double layer k = 3 + 0.3i
 // 11.0 -> 7.4 ms, modified Helmholtz single / double / hypersingular 4.20 ->
 // 3.16, 5.51 -> 4.31, 4.56 -> 3.39 ms, Laplace double layer 2.91 -> 2.80 ms.

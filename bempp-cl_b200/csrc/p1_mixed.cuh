@@ -60,9 +60,10 @@
 // memory and added to the matrix once per (test dof, trial dof)
 // (warp_cols.cuh): ~3.5x fewer FP64 L2 atomics, which bound the double-layer
 // sweep (each pair adds two blocks).
-// Issue-bound.  Double layer, 10952 elements, k = 6: 6.77 -> 5.79 ms from packing
-// neighbouring trial points to packing a vertex's two, with the Newton step of
-// the DP0 sweep; error 3.74e-8 either way.
+// Bound by latency at three CTAs per SM (168 registers; double layer: FMA pipe 55 %
+// of its cycles, issue 55 %, first stall the fixed latency).  Double layer, 10952
+// elements, k = 6: 6.77 -> 5.67 ms from packing neighbouring trial points to packing
+// a vertex's two, with the Newton step of the DP0 sweep; error 3.74e-8 either way.
 #pragma once
 
 #include <type_traits>

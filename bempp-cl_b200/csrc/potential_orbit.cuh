@@ -26,9 +26,9 @@
 //   magnetic potential   (x - c) x (alpha e_j sigma_j + gamma h0) - (e_j x gamma) sigma_j
 //   far fields           V = gamma g0 + alpha e_j tau_j, W = 2 alpha g0: ik V - x W, ik x x V.
 // The kernels they replace evaluated every source's vector terms and a range-reduced sine / cosine pair.
-// All of them are bound by the FP64 pipe.  Before -> here: Helmholtz single layer on P1, 8192 elements, 10000 points 1393 ->
-// 1321 us; electric potential, 4232 elements, 4999 points 1898 -> 541 us; electric far field, 8192 elements, 3600
-// directions 1383 -> 529 us.
+// All of them are bound by the FP64 pipe.  Before -> here: Helmholtz single layer on P1, 8192 elements, 10000 points 1396 ->
+// 1232 us; electric potential, 4232 elements, 4999 points 1903 -> 531 us; electric far field, 8192 elements, 3600
+// directions 1384 -> 490 us.
 #pragma once
 
 #include "potential.cuh"

@@ -8,15 +8,17 @@
 namespace bc {
 
 // Row blocks of the P1 and Maxwell sweeps: 32 test elements per CTA, halved while that would leave the GPU
-// under four waves of working CTAs (a symmetric sweep's CTAs below the diagonal exit at once; 3 CTAs per SM), down to
-// one.  The kernels take their chunk height as ceil(ntest / gridDim.y).  32 rows against the halved ones: single layer
+// under twelve working CTAs per SM (a symmetric sweep's CTAs below the diagonal exit at once), down to one: four waves of
+// the kernels that hold three CTAs per SM, six of those that hold two (the FP64 Maxwell fields with a real wavenumber, the
+// skew sweeps of the Helmholtz double layers).  The kernels take their chunk height as ceil(ntest / gridDim.y).  32 rows
+// against the halved ones: single layer
 // P1, 1152 elements 0.239 and 0.143 ms; electric field, 288 elements 0.094 and 0.075 ms; from 4096 elements on (P1, symmetric) the
-// launch has its four waves and keeps 32, one staging per 32 rows.
+// launch has its twelve and keeps 32, one staging per 32 rows.
 inline unsigned lin_row_blocks(int64_t ntrial, int64_t ntest, bool sym) {
     const int64_t cols = (ntrial + DP0_THREADS - 1) / DP0_THREADS;
-    const int64_t wave = (int64_t)bc_sm_count() * 3;
+    const int64_t least = 12 * (int64_t)bc_sm_count();
     int rows = 32;
-    while (rows > 1 && cols * ((ntest + rows - 1) / rows) / (sym ? 2 : 1) < 4 * wave) rows /= 2;
+    while (rows > 1 && cols * ((ntest + rows - 1) / rows) / (sym ? 2 : 1) < least) rows /= 2;
     return (unsigned)((ntest + rows - 1) / rows);
 }
 

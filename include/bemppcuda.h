@@ -109,7 +109,9 @@ typedef struct {
                            adjoint double layer and hypersingular (Helmholtz with Re k > 0, Laplace,
                            modified Helmholtz), P1 beside P0 for the scalar operators; Maxwell electric and magnetic fields (Re k > 0);
                            6-point rule.
-                           Other operators return BEMPPCUDA_ERR_UNSUPPORTED under MIXED */
+                           Other operators return BEMPPCUDA_ERR_UNSUPPORTED under MIXED.  The symmetric DP0
+                           sweeps and the P1 and Maxwell operators run in FP64 under it with a 6-point rule
+                           that is not the two-orbit one of quad_points */
     int32_t is_complex; /* result is complex128 (1) or float64 (0) */
     double params[4];   /* kernel parameters: (Re k, Im k) or (omega) */
     bemppcuda_grid test_grid;
@@ -118,14 +120,20 @@ typedef struct {
     bemppcuda_space trial; /* domain */
     int32_t grids_identical;
     int32_t nq;                 /* regular rule size <= BEMPPCUDA_MAX_REGULAR_POINTS */
-    const double *quad_points;  /* HOST (nq, 2) reference points */
+    const double *quad_points;  /* HOST (nq, 2) reference points.  The order-4 rule is recognised (to 2e-15) by
+                                   its two orbits of three points of equal weight, listed one after the other as
+                                   (a, 1 - 2a), (1 - 2a, a), (a, a).  Six points in another order or of another
+                                   rule give the same sums, without mixed precision (see precision) and, for
+                                   P1 and Maxwell operators with a complex wavenumber, modified Helmholtz, the
+                                   Laplace double layers and the Helmholtz hypersingular operator, by the
+                                   general kernel, several times slower */
     const double *quad_weights; /* HOST (nq,) */
     void *result;               /* (rows, ld) row-major float64 or complex128 */
     int64_t ld;                 /* row stride in entries */
     int32_t overwrite;          /* DP0 fast path only: store instead of add, zero for adjacent pairs */
     int32_t no_symmetry;        /* 0: when test and trial are the same space of one grid (same support, dof
                                    map, multiplier, normal-multiplier and geometry pointers; DP0, P1 / DP1 /
-                                   P0, RWG with SNC) and k is real, one sweep over the pairs i < j gives
+                                   P0, RWG with SNC), one sweep over the pairs i < j gives
                                    A_ij and A_ji; 1: always evaluate every entry separately */
     double phase_radius;        /* R_test + R_trial, R = largest centroid-to-vertex distance of a grid;
                                    lets the mixed path skip the phase range reduction when
@@ -185,7 +193,8 @@ typedef struct {
                                       use a rule that is symmetric under exchanging test and trial points
                                       (the vertex-adjacent rule), so the pair with test < trial adds both
                                       entries (blocks) and its reverse adds nothing -- DP0 scalar kernels,
-                                      and on P1 x P1 the single layers and hypersingular operators; 0 = off */
+                                      and on P1 x P1 the single layers and hypersingular operators; at order 4
+                                      of bemppcuda_assemble_singular_duffy every kernel; 0 = off */
 } bemppcuda_singular_args;
 
 /* Potential / far-field evaluation (numba_kernels.py:1788-1849, 2281-2570). */
