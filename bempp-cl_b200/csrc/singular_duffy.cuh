@@ -354,6 +354,9 @@ __device__ __forceinline__ void duffy_group(const DuffyTarget &prm, const DuffyT
     const int kind = npts == SD_SAME * SD_Q ? 0 : npts == SD_EDGE * SD_Q ? 1 : 2;
     const bool mirror = prm.mirror && !prm.values && kind == 2;
     if (mirror && t > s) valid = false;
+    // the magnetic field of a coincident pair is zero (all its vectors lie in one plane), where the rounding of its sums,
+    // each of them large, would be 5e-14 of the matrix
+    if (ASM == BEMPPCUDA_ASM_MFIE && kind == 0) valid = false;
     const double kr = prm.p[0], ki = CK ? prm.p[1] : 0.0;
     Geom gt, gs;
     DuffyOrder ot = {}, os = {};

@@ -132,10 +132,9 @@ def test_other_orders_take_the_tables(oracle, case, order):
     assert float(torch.linalg.vector_norm(parts[0] - parts[1]) / np.linalg.norm(ref)) < 1e-12
 
 
-@pytest.mark.parametrize("equation,name,kind,degree", [CASES[1], CASES[5], CASES[8], CASES[12], CASES[13]])
-def test_values_per_pair(equation, name, kind, degree):
-    """The pairs' blocks in the caller's array instead of a matrix, added to what is there."""
-    from bempp_cuda import _lib, operators
+def _values(equation, name, kind, degree, structured):
+    """The pairs' blocks in the caller's array instead of a matrix, added to the ones that are there; and the pairs."""
+    from bempp_cuda import _lib
     from bempp_cuda.assembly import _set_params, kernel_ids, result_dtype
     from bempp_cuda.device import current_stream, device_grid, device_singular_rule, device_space
     from bempp_cuda.shapes import ellipsoid
@@ -146,23 +145,35 @@ def test_values_per_pair(equation, name, kind, degree):
     dual = function_space(grid, "SNC", 0) if kind == "RWG" else domain
     d = _descriptor(equation, name, domain, dual, 1.5)
     rule = device_singular_rule(grid, 4, dual.support, domain.support)
-    shapes = device_space(dual).nshape * device_space(domain).nshape
-    lib, out = _lib.load(), []
-    for entry in (lambda a: lib.bemppcuda_assemble_singular_duffy(a, 4, current_stream()),
-                  lambda a: lib.bemppcuda_assemble_singular(a, current_stream())):
-        args = _lib.SingularArgs()
-        args.kernel, args.assembly = kernel_ids(d)
-        args.is_complex = 1 if d.is_complex else 0
-        _set_params(args, d.options)
-        args.grid, args.test, args.trial = (device_grid(grid).record(), device_space(dual).record(),
-                                            device_space(domain).record())
-        rule.fill(args)
-        args.phase_radius = 1.0001 * 2.0 * device_grid(grid).radius
-        values = torch.ones(rule.npairs * shapes, dtype=result_dtype(d), device="cuda")
-        args.values = values.data_ptr()
-        _lib.check(entry(args))
-        out.append(values - 1.0)
-    assert float(torch.linalg.vector_norm(out[1])) > 0.0
+    args = _lib.SingularArgs()
+    args.kernel, args.assembly = kernel_ids(d)
+    args.is_complex = 1 if d.is_complex else 0
+    _set_params(args, d.options)
+    args.grid, args.test, args.trial = (device_grid(grid).record(), device_space(dual).record(),
+                                        device_space(domain).record())
+    rule.fill(args)
+    args.phase_radius = 1.0001 * 2.0 * device_grid(grid).radius
+    shapes = (device_space(dual).nshape, device_space(domain).nshape)
+    values = torch.ones((rule.npairs,) + shapes, dtype=result_dtype(d), device="cuda")
+    args.values = values.data_ptr()
+    lib = _lib.load()
+    _lib.check(lib.bemppcuda_assemble_singular_duffy(args, 4, current_stream()) if structured
+               else lib.bemppcuda_assemble_singular(args, current_stream()))
+    return values - 1.0, rule
+
+
+@pytest.mark.parametrize("equation,name,kind,degree", [CASES[1], CASES[5], CASES[8], CASES[12], CASES[13]])
+def test_values_per_pair(equation, name, kind, degree):
+    got, ref = (_values(equation, name, kind, degree, structured)[0] for structured in (True, False))
+    assert float(torch.linalg.vector_norm(ref)) > 0.0
     tol = 1e-12 if "double" in name or name == "magnetic_field" else 1e-13
     # (adding to one loses eps per value)
-    assert float((out[0] - out[1]).abs().max()) < tol * float(out[1].abs().max()) + 4e-16
+    assert float((got - ref).abs().max()) < tol * float(ref.abs().max()) + 4e-16
+
+
+@pytest.mark.parametrize("equation,name,kind,degree", [CASES[6], CASES[13]])
+def test_coincident_blocks_in_one_plane_are_zero(equation, name, kind, degree):
+    """Double layers and the magnetic field of an element with itself."""
+    got, rule = _values(equation, name, kind, degree, True)
+    assert float(got[rule.test_elements == rule.trial_elements].abs().max()) == 0.0
+    assert float(got.abs().max()) > 0.0
